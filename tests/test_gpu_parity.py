@@ -141,7 +141,7 @@ def test_single_grain_full_size_against_fp64_oracle():
     plain = _sim(sc0)
     for _ in range(10):
         plain.step()
-    grain_checks(sc0, plain, err, o, 10, "grain_40")
+    grain_checks(sc0, plain, err, o, 10, "grain_full_10")
     plain.close()
 
 
