@@ -66,15 +66,17 @@ typedef struct {
     int precision;          /* 0: FP32 state; 1: FP32 bulk + compensated hi/lo
                                position and velocity in predictor/corrector          */
     int max_secant_iter;    /* Johnson-Cook secant limit (plasticity.cuh:66: 100)     */
-    int lanes_per_particle; /* pair-loop tiling: 8, 16 or 32 lanes of a warp per
-                               particle; 0 picks the tuned default                   */
+    int lanes_per_particle; /* 0, 8, 16 or 32, kept for callers that set it: the pair
+                               loop has one mapping of lanes to particles and ignores
+                               the value                                              */
     int diagnostics;        /* 1: keep neighbour counts, half-step positions and
                                contact normals for mfree_get_field()                  */
     int friction_tool_vel;  /* 1: subtract the tool velocity in the friction slip
                                velocity.  The reference never uploads its tool_vel
                                constant (tool_3d_gpu.cu:26,528), so 0 matches it.    */
-    int tile_depth;         /* pair-loop tiling: cells per tile along z, 1..8; 0 picks
-                               the tuned default (6).  Results do not depend on it.   */
+    int tile_depth;         /* pair-loop tiling: most cells of a tile along z, 1..8; 0
+                               picks the default (8; tiles are cut by their particle
+                               count within it).  Results do not depend on it.        */
     int full_stencil;       /* 1: the pair loop visits every candidate of the 5x5x5
                                cell stencil and evaluates every term.  0 (default):
                                it skips the stencil cells that lie wholly beyond the
@@ -370,7 +372,7 @@ int mfree_cell_list_static(const float *pos4, int n, const float bbmin[3], float
  * of any sizes (each an mfree_ctx, configured as for mfree_step) and steps
  * all of them with one launch per kernel: every scene keeps its own state and
  * cell list, and a scene's results are the same alone and in a batch when the
- * pair-loop tiling is the same.  Scenes are admitted and retired between
+ * pair-loop tiling is the same (and whatever it is).  Scenes are admitted and retired between
  * steps (continuous batching): admission is bounded by a device-memory
  * budget, and a scene may be admitted with a step count after which it stops.
  * All scenes of a batch share the pair-kernel variant (cspm, conduction,
@@ -405,11 +407,11 @@ int mfree_batch_context(mfree_batch *b, int slot, mfree_ctx **ctx);
 int mfree_batch_retire(mfree_batch *b, int slot, mfree_ctx **ctx);
 /* scenes held, running scenes, device bytes held by them and the budget */
 int mfree_batch_info(mfree_batch *b, int *scenes, int *running, size_t *bytes, size_t *budget);
-/* Pair-loop tiling of the batch: lanes per particle (8, 16, 32) and tile depth
- * (1..8 cells); 0 keeps the current value. */
+/* Pair-loop tiling of the batch: lanes per particle (8, 16, 32; without effect)
+ * and the largest tile depth (1..8 cells); 0 keeps the current value. */
 int mfree_batch_set_tiling(mfree_batch *b, int lanes_per_particle, int tile_depth);
 int mfree_batch_get_tiling(mfree_batch *b, int *lanes_per_particle, int *tile_depth);
-/* Autotuner: times every tiling (lanes per particle x tile depth 4..8) for
+/* Autotuner: times every largest tile depth (4..8) for
  * trial_steps steps on copies of the batch's running scenes (their own state
  * is untouched) and keeps the fastest.  The cell size stays the reference's
  * (the smoothing length), which the bit-exact cell ids and order require.

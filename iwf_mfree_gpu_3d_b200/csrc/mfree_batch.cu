@@ -46,7 +46,7 @@ struct mfree_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int device = 0, num_sms = 148;
-    int lpp = 8, tile_z = 6;
+    int lpp = 8, tile_z = TILE_Z_MAX;
     bool variant_set = false, cspm = false, prec = false;
     int cond = 0;
     std::vector<Slot> slots;
@@ -54,10 +54,10 @@ struct mfree_batch {
     void *d_table = nullptr;
     int cap = 0;
     int2 *d_tiles = nullptr;  // the pair kernel's tile list over every scene
-    int tiles_cap = 0;
+    long long tiles_cap = 0;
     BatchTable T{};
     std::vector<int> run;  // slots in the table, in table order
-    int tot_pblk = 0, tot_stile = 0, tot_cblk = 0, tot_itile = 0;
+    int tot_pblk = 0, tot_stile = 0, tot_cblk = 0, tot_ibun = 0;
     bool dirty = true;
     int table_record_every = -1;
     cudaGraphExec_t graph = nullptr;
@@ -103,12 +103,15 @@ int build_table(mfree_batch *b, int record_every) {
     b->T.pblk = dint;
     b->T.stile = dint + (b->cap + 1);
     b->T.cblk = dint + 2 * (b->cap + 1);
-    b->T.itile = dint + 3 * (b->cap + 1);
+    b->T.ibun = dint + 3 * (b->cap + 1);
     b->T.tile_next = dint + 4 * (b->cap + 1);
     b->T.tile_count = dint + 4 * (b->cap + 1) + 1;
     std::vector<StepArgs> args(2 * size_t(n));
     std::vector<int> pre(4 * size_t(b->cap + 1), 0);
     int *pb = pre.data(), *ps = pb + (b->cap + 1), *pc = ps + (b->cap + 1), *pt = pc + (b->cap + 1);
+    long long particles = 0, tiles = 0;
+    for (int k : b->run) particles += b->slots[k].c->n_init;
+    const int cap_targets = default_tile_cap(particles, b->num_sms);
     for (int s = 0; s < n; s++) {
         Slot &sl = b->slots[b->run[s]];
         mfree_ctx *c = sl.c;
@@ -125,6 +128,7 @@ int build_table(mfree_batch *b, int record_every) {
             StepArgs a = make_args(c);
             a.p.record_every = record_every;
             a.p.tile_z = b->tile_z;
+            a.p.tile_cap = cap_targets;
             args[2 * s + p] = a;
         }
         c->cur = keep;
@@ -132,15 +136,16 @@ int build_table(mfree_batch *b, int record_every) {
         pb[s + 1] = pb[s] + hash_blocks(c);
         ps[s + 1] = ps[s] + scan_tiles(c);
         pc[s + 1] = pc[s] + int((c->num_cell + 255) / 256);
-        pt[s + 1] = pt[s] + num_tiles(P);
+        pt[s + 1] = pt[s] + num_bundles(P);
+        tiles += max_tiles(P);
     }
     b->tot_pblk = pb[n];
     b->tot_stile = ps[n];
     b->tot_cblk = pc[n];
-    b->tot_itile = pt[n];
-    if (b->tot_itile > b->tiles_cap) {  // the tile list of all scenes
+    b->tot_ibun = pt[n];
+    if (tiles > b->tiles_cap) {  // the tile list of all scenes
         CUDA_TRY(cudaStreamSynchronize(b->stream));  // the old list may still be read
-        const int cap = std::max(b->tot_itile, 2 * b->tiles_cap);
+        const long long cap = std::max(tiles, 2 * b->tiles_cap);
         if (b->d_tiles) cudaFree(b->d_tiles);
         b->d_tiles = nullptr;
         b->tiles_cap = 0;
@@ -152,7 +157,7 @@ int build_table(mfree_batch *b, int record_every) {
     // vectors may go; the device copy stays ordered on the stream
     CUDA_TRY(cudaMemcpyAsync(dargs, args.data(), sizeof(StepArgs) * args.size(), cudaMemcpyHostToDevice, b->stream));
     CUDA_TRY(cudaMemcpyAsync(dint, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, b->stream));
-    cudaError_t e = launch_interact_batch(b->T, b->lpp, b->cspm, b->cond, b->prec, 0, b->stream);
+    cudaError_t e = launch_interact_batch(b->T, b->cspm, b->cond, b->prec, 0, b->stream);
     if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("batched pair kernel setup: ") + cudaGetErrorString(e));
     return MFREE_OK;
 }
@@ -170,9 +175,9 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     kb_scan_top<<<n, 1024, 0, s>>>(T);
     kb_scan_down<<<b->tot_stile, SCAN_THREADS, 0, s>>>(T);
     kb_scatter<<<b->tot_pblk, HASH_BLOCK, 0, s>>>(T);
-    kb_cell_fixup<<<b->tot_cblk + (b->tot_itile + 255) / 256, 256, 0, s>>>(T);
+    kb_cell_fixup<<<b->tot_cblk + (b->tot_ibun + 7) / 8, 256, 0, s>>>(T);
     cudaError_t e = launch_gather_predict_batch(T, b->prec, b->tot_pblk, s);
-    if (e == cudaSuccess) e = launch_interact_batch(T, b->lpp, b->cspm, b->cond, b->prec, b->num_sms, s);
+    if (e == cudaSuccess) e = launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s);
     if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));
     kb_finalize<<<b->tot_pblk, 256, 0, s>>>(T);
     kb_force_final<<<n, 256, 0, s>>>(T);
@@ -442,8 +447,7 @@ int mfree_batch_autotune(mfree_batch *b, int trial_steps, int *lpp_out, int *tz_
     CUDA_TRY(cudaEventCreate(&e1));
     double best = 1e300;
     int blpp = b->lpp, btz = b->tile_z;
-    const int lpps[] = {8, 16, 32};
-    for (int lpp : lpps)
+    const int lpp = 8;  // the pair kernel has one mapping of lanes to particles
         for (int tz = 4; tz <= TILE_Z_MAX && !st; tz++) {
             if ((st = mfree_batch_set_tiling(tb, lpp, tz))) break;
             if ((st = mfree_batch_step(tb, 1, 0, 1))) break;  // capture + warm-up

@@ -116,7 +116,7 @@ struct mfree_ctx {
     // one-scene table of the batched kernels (ensure_table)
     unsigned char *d_table = nullptr;
     int2 *d_tiles = nullptr;  // the pair kernel's list of non-empty tiles (grid-sized scratch)
-    int ntiles = 0;           // tiles of the grid at the table's depth
+    int nbun = 0;             // bundles of tiles of the grid
     mfree::BatchTable T{};
     unsigned long long table_version = ~0ull;
     int table_record_every = -1;
@@ -136,6 +136,7 @@ namespace host {
 
 int default_lpp();
 int default_tile_depth();
+int default_tile_cap(long long n, int num_sms);
 int hash_blocks(const mfree_ctx *c);
 int scan_tiles(const mfree_ctx *c);
 StepArgs make_args(mfree_ctx *c);

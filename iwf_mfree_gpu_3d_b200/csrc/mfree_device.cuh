@@ -21,8 +21,9 @@
 //   contiguous range of each of the two, staged into shared memory by two bulk
 //   copies:
 //     P = (x, y, z, tool_flag)      V = (vx, vy, vz, rho)
-//     A = sigma(xx, yy, zz, xy)     B = (sigma_xz, sigma_yz, c = sqrt(K/rho), h)
-//     R = R(xx, yy, zz, xy)         C = (R_xz, R_yz, T, m/rho)
+//     A = sigma(xx, xy, xz, yz)     B = (sigma_yy, sigma_zz, c = sqrt(K/rho), h)
+//     R = R(xx, xy, xz, yz)         C = (R_yy, R_zz, T, m/rho)
+//   (the order in which the pair body's packed arithmetic takes them as pairs)
 //   with sigma = (S - p I)/rho^2 (the per-particle factor of the stress
 //   divergence, interactions_gpu.cu:389-399) and R the artificial stress.
 #pragma once
@@ -128,7 +129,8 @@ struct Params {
     int num_tools;
     float tool0_vel[3];  // global_tool[0]->get_vel(): friction heat and tool particles
     int record_every;
-    int tile_z;  // cells per pair-kernel tile along z (1..TILE_Z_MAX)
+    int tile_z;    // largest depth of a pair-kernel tile (cells along z, 1..TILE_Z_MAX)
+    int tile_cap;  // targets a tile should hold at most
     int stage_extra;  // bytes added to the staging byte count: nonzero only to make the waits run out (tests)
     int full_stencil;  // 1: the pair kernel visits every stencil candidate (no geometric pruning)
 };

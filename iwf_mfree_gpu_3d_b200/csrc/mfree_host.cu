@@ -95,7 +95,20 @@ void invalidate_graphs(mfree_ctx *c) {
 }
 
 int default_lpp() { return 8; }
-int default_tile_depth() { return 6; }
+int default_tile_depth() { return TILE_Z_MAX; }
+// Targets a tile should hold.  A block serves 240 at once (mfree_interact.cuh),
+// a tile comes out about 70 % full (levels of a bundle are not divided, bundles
+// at a surface are thin), and its time is mostly that of one target's chain: so
+// as full as possible for many particles, and for few as small as fills the
+// waves of blocks they need at least.  Measured, pair kernel in us at 64 / 128 /
+// 160 / 192 / 240 targets: 8,000 particles 60 / 51 / 53 / 54 / 59 (46 at the
+// rule's 77); 30,597 with CSPM + PSE 131 / 103 / 94 / 101 / 128; 252,000
+// 689 / 437 / 395 / 360 / 356; 1M with CSPM + PSE 3108 / 1850 / 1640 / 1494 / 1378.
+int default_tile_cap(long long n, int num_sms) {
+    const double fill = 0.7;
+    const long long waves = (long long)std::ceil(double(n) / (240 * fill * num_sms));
+    return std::min(240, std::max(32, int(double(n) / (double(std::max<long long>(waves, 1)) * num_sms * fill))));
+}
 
 Params make_params(const mfree_ctx *c) {
     Params P{};
@@ -160,6 +173,7 @@ Params make_params(const mfree_ctx *c) {
     for (int d = 0; d < 3; d++) P.tool0_vel[d] = c->tools.empty() ? 0.f : c->tools[0]->vel[d];
     P.record_every = 0;
     P.tile_z = c->opt.tile_depth > 0 ? c->opt.tile_depth : default_tile_depth();
+    P.tile_cap = default_tile_cap(c->n_init, c->num_sms);
     P.stage_extra = c->inject_staging ? 16 : 0;
     return P;
 }
@@ -274,8 +288,8 @@ int ready(mfree_ctx *c) {
     if (st) return st;
     {
         const StepArgs a = make_args(c);
-        cudaError_t e = launch_interact_batch(BatchTable{}, lpp ? lpp : default_lpp(), a.p.cspm != 0, a.p.conduction,
-                                              a.p.precision != 0, 0, c->stream);
+        cudaError_t e = launch_interact_batch(BatchTable{}, a.p.cspm != 0, a.p.conduction, a.p.precision != 0, 0,
+                                              c->stream);
         if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("pair kernel setup: ") + cudaGetErrorString(e));
     }
     if (c->clock_dirty) return write_clock(c);
@@ -314,8 +328,8 @@ int ensure_table(mfree_ctx *c, int record_every) {
     }
     c->cur = keep;
     const Params &P = args[0].p;
-    const int ntiles = num_tiles(P);
-    const int pre[10] = {0, hash_blocks(c), 0, scan_tiles(c), 0, int((c->num_cell + 255) / 256), 0, ntiles, 0, 0};
+    const int nbun = num_bundles(P);
+    const int pre[10] = {0, hash_blocks(c), 0, scan_tiles(c), 0, int((c->num_cell + 255) / 256), 0, nbun, 0, 0};
     StepArgs *da = (StepArgs *)c->d_table;
     int *di = (int *)(da + 2);
     // pageable sources: the call returns once the bytes are staged
@@ -325,12 +339,12 @@ int ensure_table(mfree_ctx *c, int record_every) {
     c->T.pblk = di;
     c->T.stile = di + 2;
     c->T.cblk = di + 4;
-    c->T.itile = di + 6;
+    c->T.ibun = di + 6;
     c->T.tile_next = di + 8;
     c->T.tile_count = di + 9;
     c->T.tile_list = c->d_tiles;
     c->T.nscenes = 1;
-    c->ntiles = ntiles;
+    c->nbun = nbun;
     c->table_version = c->version;
     c->table_record_every = record_every;
     return MFREE_OK;
@@ -346,7 +360,6 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     cudaStream_t s = c->stream;
     const int hb = hash_blocks(c), tiles = scan_tiles(c);
     const int nb = (c->n_init + 255) / 256;
-    const int lpp = c->opt.lanes_per_particle ? c->opt.lanes_per_particle : default_lpp();
     cudaError_t le = cudaSuccess;
     auto run = [&](int id, auto &&launch) {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -368,10 +381,10 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     run(3, [&] { kb_scan_top<<<1, 1024, 0, s>>>(T); });
     run(4, [&] { kb_scan_down<<<tiles, SCAN_THREADS, 0, s>>>(T); });
     run(5, [&] { kb_scatter<<<hb, HASH_BLOCK, 0, s>>>(T); });
-    run(6, [&] { kb_cell_fixup<<<int((c->num_cell + 255) / 256) + (c->ntiles + 255) / 256, 256, 0, s>>>(T); });
+    run(6, [&] { kb_cell_fixup<<<int((c->num_cell + 255) / 256) + (c->nbun + 7) / 8, 256, 0, s>>>(T); });
     run(7, [&] { le = launch_gather_predict_batch(T, P.precision != 0, nb, s); });
     if (le == cudaSuccess)
-        run(8, [&] { le = launch_interact_batch(T, lpp, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
+        run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
     if (le != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(le));
     run(9, [&] { kb_finalize<<<nb, 256, 0, s>>>(T); });
     if (!c->tools.empty()) run(10, [&] { kb_force_final<<<1, 256, 0, s>>>(T); });
@@ -1374,7 +1387,7 @@ int get_field_impl(mfree_ctx *c, int f, float *fo, double *dout) {
             std::vector<Rec> R;
             if ((st = copy_records(c, R))) return st;
             for (int i = 0; i < n; i++) {
-                float s6[6] = {R[i].R.x, R[i].R.y, R[i].R.z, R[i].R.w, R[i].C.x, R[i].C.y};
+                float s6[6] = {R[i].R.x, R[i].C.x, R[i].C.y, R[i].R.y, R[i].R.z, R[i].R.w};  // xx yy zz xy xz yz
                 sym_to_9(s6, &tmp[size_t(i) * 9]);
             }
             break;

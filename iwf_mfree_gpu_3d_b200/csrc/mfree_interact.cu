@@ -4,9 +4,8 @@
 
 namespace mfree {
 
-cudaError_t launch_interact_batch(const BatchTable &T, int lpp, bool cspm, int cond, bool prec, int grid,
-                                  cudaStream_t s) {
-    return with_lpp(lpp, cspm, cond, prec, [&](auto v) { return decltype(v)::batch(T, grid, s); });
+cudaError_t launch_interact_batch(const BatchTable &T, bool cspm, int cond, bool prec, int grid, cudaStream_t s) {
+    return with_variant(cspm, cond, prec, [&](auto v) { return decltype(v)::batch(T, grid, s); });
 }
 
 }  // namespace mfree

@@ -14,27 +14,36 @@
 //                             leap_frog.cu:102-119, actions_gpu.cu:55-68,451-487
 //                             (particles inside a tool box defer these to kb_finalize)
 //
-// Work decomposition: a persistent block (640 threads, one per SM) pulls
-// tiles of 4 x 4 x D cells (D = Params::tile_z, 6 by default) of every scene
-// of the table from one work counter.  The tile's particles are 16 contiguous
-// ranges of the sorted order; the records their 5x5x5 stencils touch are the
-// 64 contiguous column ranges of the 8 x 8 x (D+4)-cell halo, staged into
-// shared memory with two bulk copies per column, its P records and the
-// interleaved rest (TMA cp.async.bulk, completion counted on an mbarrier,
-// bounded waits).  Each
-// target is served by a group of LPP lanes.  Pass A streams the target's
-// candidates (25 column ranges of the staged halo) through the lanes: support
-// test, PSE (which sums every stencil candidate) and a ballot that compacts
-// the in-support neighbours into a queue.  The CSPM pass (symmetric matrix)
-// and the pair pass run on the queue only -- the reference evaluates the pair
-// body for every candidate, ~3.5x more work, and candidates outside the
-// support contribute exact zeros there.  Accumulators are reduced across the
-// group with xor shuffles; then one thread per target runs the per-particle
-// epilogue.  The epilogue needs at most TCAP = 320 threads; during the
-// epilogue of a tile's last pass the other 320 already prepare the next tile
-// (its target ranges, halo table and staging copies), so those copies land
-// while the epilogue runs.
+// Work decomposition: a persistent block (one per SM) pulls tiles of 4 x 4 x D
+// cells (D up to 8) of every scene of the table from one work
+// counter (the tile list cuts the grid so that tiles are about equally full).
+// The tile's particles are 16 contiguous ranges of the sorted order;
+// the records their 5x5x5 stencils touch are the 64 contiguous column ranges
+// of the 8 x 8 x (D+4)-cell halo, staged into shared memory with two bulk
+// copies per column, its P records and the interleaved rest (TMA
+// cp.async.bulk, completion counted on an mbarrier, bounded waits).
+//
+// Two lanes serve a target; the 512 compute threads hold up to 256 targets of
+// a tile at once, each from its candidates to its new state without a barrier
+// in between.  The candidate pass walks the 25 stencil columns of the target's
+// cell, the two lanes on alternate records, and puts the in-support neighbours
+// into a queue that the lanes fill from its two ends.  The pair pass runs on
+// the queue only -- the reference evaluates the pair body for every candidate,
+// ~3.5x more work, and candidates outside the support contribute exact zeros
+// there.  One shuffle per sum joins the two lanes, then the first runs the
+// fused rest of the step.  A producer warp builds the next tile's tables
+// while the compute warps work, and issues its copies as soon as they have
+// read the last record of the current tile, so that the copies land while the
+// epilogue runs.
+//
+// The kernel is bound by instruction issue, not by the FP32 pipe or memory:
+// the split follows from the instructions it saves.  Eight lanes a target (an
+// earlier form) spent about 80 instruction slots a candidate on ballots and on
+// walking columns that are about as long as the group is wide, and reduced 25
+// sums over 8 lanes.
 #pragma once
+
+#include <type_traits>
 
 #include "mfree_kernels.cuh"
 
@@ -57,100 +66,345 @@ __device__ __forceinline__ void inv3s(const float *m, float det, float *o) {
     o[5] = (m[3] * m[4] - m[0] * m[5]) * id;  // yz
 }
 
-// the target's terms of the pair loop; its own sigma and R enter the stress
-// divergence only through the group's sums (see pair_body) and are read after
-// the loop
-struct IData {
-    float x, y, z, vx, vy, vz, rho, c, h, T, tool;
-    float h1, fac;
-};
-
-// gradient factor of cubic_spline (kernels.cuh:26-69): value w and
-// dfac = der*fac with grad W = dfac * (x_i - x_j)
-__device__ __forceinline__ void spline(float r2, float h1, float fac, float &w, float &dfac) {
-    float rinv;  // r2 >= 1e-8 here: never a denormal
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(r2));
-    const float r = r2 * rinv;
-    const float q = r * h1;
-    float val, der;
-    if (q > 1.f) {
-        const float t = 2.f - q, t2 = t * t;
-        val = 0.25f * t2 * t;
-        der = -0.75f * t2 * h1 * rinv;
-    } else {
-        val = 1.f - 1.5f * q * q * (1.f - 0.5f * q);
-        der = -3.0f * q * (1.f - 0.75f * q) * h1 * rinv;
-    }
-    w = val * fac;
-    dfac = der * fac;
+// ------------------------------------------------------ packed arithmetic --
+// two FP32 operations per instruction (FADD2/FMUL2/FFMA2): the same IEEE
+// results as two scalar ones, half the issue slots
+__device__ __forceinline__ unsigned long long f2_bits(float2 v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+    return r;
+}
+__device__ __forceinline__ float2 f2_of(unsigned long long r) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+    return v;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+    return f2_of(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_of(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_of(d);
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-// the scene constants of the pair body, held in registers for a target's
-// pair loop (read from the shared-memory arguments in the loop they were
-// loaded again for every pair: 1.869 -> 1.847 ms on the 1M step)
-struct PairConst {
-    float inv_wdeltap, eta2, alpha, beta;  // 1 / wdeltap, eta^2 (as eta * eta), AV alpha and beta
-    bool art;                              // artificial stress on (wdeltap > 0)
+// -------------------------------------------------------------- pair body --
+// the target's terms of the pair loop; its own sigma and R enter the stress
+// divergence only through the sums (see finish_sums) and are read after the
+// loop.  Differences and sums are packed with an addition each, so the
+// target's values are kept with the sign they are added with.
+struct Target {
+    float2 nxy;       // -x, -y
+    float nz;         // -z
+    float2 nvxy;      // -vx, -vy
+    float2 nvz_rho;   // -vz, rho
+    float2 ch;        // c, h
+    float T, tool, h1;
+    float c_art;      // W(0-free part) factor / wdeltap: fab = (val c_art)^4
+    bool art;
 };
-template <bool CSPM, int COND>
-__device__ __forceinline__ void pair_body(const PairConst &P, const IData &I, const float *invB, const float4 Pj,
-                                          const float4 Vj, const float4 Aj, const float4 Bj, const float4 Rj,
-                                          const float4 Cj, float *acc) {
-    const float dx = I.x - Pj.x, dy = I.y - Pj.y, dz = I.z - Pj.z;
-    const float r2 = dist2_rn(dx, dy, dz);
-    float w, dfac;
-    spline(r2, I.h1, I.fac, w, dfac);
-    float gx = dfac * dx, gy = dfac * dy, gz = dfac * dz;
-    if (CSPM) {
-        const float ux = gx * invB[0] + gy * invB[3] + gz * invB[4];
-        const float uy = gx * invB[3] + gy * invB[1] + gz * invB[5];
-        const float uz = gx * invB[4] + gy * invB[5] + gz * invB[2];
-        gx = ux; gy = uy; gz = uz;
+// the scene's constants of the pair body, in registers for a target's loop
+struct PairConst {
+    float eta2_4, alpha_2, beta_2;  // eta^2 / 4, -AV alpha / 2, AV beta / 2
+};
+
+// The sums of a target.  Every gradient sum is taken with the pair's unscaled
+// factor g = (u^2 - t^2/4)/r (x_i - x_j), t = 2 - q, u = max(1 - q, 0), q = r/h:
+// grad W = 3 fac/h g with fac = 1/(pi h^3), and W = fac (t^3/4 - u^3) (the two
+// branches of cubic_spline, kernels.cuh:26-69, in one expression).  The factor
+// and, with CSPM, the correction matrix are applied once after the loop: all
+// terms are linear in the gradient.  So CSPM needs no pass of its own over the
+// neighbours; the stress divergence then keeps sigma_j (x) g uncontracted.
+template <bool CSPM, int COND> struct Sums {
+    float2 Lx, Ly, Lz;       // sum vol dv_{x,y} g_x, g_y, g_z
+    float2 Lw;               // sum vol dv_z g_{x,y}
+    float Lzz;               // sum vol dv_z g_z
+    float2 s0[3], s1[3], s2[3];  // CSPM: sum (t_xx, t_xy), (t_xz, t_yz), (t_yy, t_zz) times g_x, g_y, g_z
+    float2 dx2;              // else: t_xx g_x, t_xy g_y (added: row x)
+    float2 dz2;              //       t_xz g_x, t_yz g_y (added: row z)
+    float2 dxy;              //       t_xz g_z, t_yz g_z (rows x and y)
+    float dy, dz;            //       t_xy g_x + t_yy g_y, t_zz g_z
+    float2 av; float avz;    // sum -pi_ij g
+    float2 xs; float xsz;    // sum -W/(fac rho_ij) dv / 2 (factors after the loop)
+    float2 g; float gz;      // sum g
+    float2 f; float fz;      // sum fab g
+    float2 b0; float2 b1; float bxz, bzz;  // CSPM: -sum vol d (x) g: (xx, xy), (yy, yz), xz, zz
+    float2 h0; float2 h1; float hxz, hzz;  // CSPM + Brookshaw: the heat sum before its contraction
+    float heat;              // Brookshaw without CSPM
+    __device__ __forceinline__ void zero() {
+        const float2 z = make_float2(0.f, 0.f);
+        Lx = Ly = Lz = Lw = z; Lzz = 0.f;
+#pragma unroll
+        for (int k = 0; k < 3; k++) s0[k] = s1[k] = s2[k] = z;
+        dx2 = dz2 = dxy = z; dy = dz = 0.f;
+        av = xs = g = f = z; avz = xsz = gz = fz = 0.f;
+        b0 = b1 = z; bxz = bzz = 0.f;
+        h0 = h1 = z; hxz = hzz = 0.f;
+        heat = 0.f;
     }
-    const bool mech = !(I.tool == 1.f) && !(Pj.w == 1.f);
-    const float volj = Cj.w;
-    if (mech) {
-        const float dvx = Vj.x - I.vx, dvy = Vj.y - I.vy, dvz = Vj.z - I.vz;
-        const float ax = dvx * volj, ay = dvy * volj, az = dvz * volj;
-        acc[0] = fmaf(ax, gx, acc[0]); acc[1] = fmaf(ax, gy, acc[1]); acc[2] = fmaf(ax, gz, acc[2]);
-        acc[3] = fmaf(ay, gx, acc[3]); acc[4] = fmaf(ay, gy, acc[4]); acc[5] = fmaf(ay, gz, acc[5]);
-        acc[6] = fmaf(az, gx, acc[6]); acc[7] = fmaf(az, gy, acc[7]); acc[8] = fmaf(az, gz, acc[8]);
+    // the sums as a list (zeros past COUNT), and back
+    static constexpr int COUNT = CSPM ? (COND == MFREE_COND_BROOKSHAW ? 51 : 45) : (COND == MFREE_COND_BROOKSHAW ? 25 : 24);
+    template <class F> __device__ __forceinline__ void each(F &&v) {
+        auto v2 = [&](float2 &p) { v(p.x); v(p.y); };
+        v2(Lx); v2(Ly); v2(Lz); v2(Lw); v(Lzz);
+        v2(av); v(avz); v2(xs); v(xsz); v2(g); v(gz); v2(f); v(fz);
+        if (CSPM) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) { v2(s0[k]); v2(s1[k]); v2(s2[k]); }
+            v2(b0); v2(b1); v(bxz); v(bzz);
+        } else {
+            v(dx2.x); v(dy); v(dz);
+        }
+        if (COND == MFREE_COND_BROOKSHAW) {
+            if (CSPM) { v2(h0); v2(h1); v(hxz); v(hzz); }
+            else v(heat);
+        }
+    }
+    // without CSPM: the parts of the stress divergence in one value a row
+    __device__ __forceinline__ void fold() {
+        if (CSPM) return;
+        dx2.x += dx2.y + dxy.x;
+        dy += dxy.y;
+        dz += dz2.x + dz2.y;
+        dx2.y = dxy.x = dxy.y = dz2.x = dz2.y = 0.f;
+    }
+    // the sums over the LANES lanes of a group, left in row[0..COUNT) (shared
+    // memory): a butterfly that halves the list at every step, so a lane ends
+    // with an eighth of it.  Every lane of the warp calls it.
+    template <int LANES> __device__ __forceinline__ void reduce_to(float *row, int l, bool store) {
+        fold();
+        constexpr int REST = COUNT % 8 <= 2 ? COUNT % 8 : 0;  // few left over: reduced in full
+        constexpr int MAIN = (COUNT - REST + 7) / 8 * 8;
+        float a[MAIN + 8];
+#pragma unroll
+        for (int k = 0; k < MAIN + 8; k++) a[k] = 0.f;
+        int n = 0;
+        each([&](float &v) { a[n++] = v; });
+        constexpr int STEPS = LANES == 8 ? 3 : 1;
+        int base = 0;
+#pragma unroll
+        for (int st = 0; st < STEPS; st++) {
+            const int o = LANES >> (st + 1), half = MAIN >> (st + 1);
+            const bool up = (l & o) != 0;
+            if (up) base += half;
+#pragma unroll
+            for (int k = 0; k < half; k++) {
+                const float send = up ? a[k] : a[k + half], keep = up ? a[k + half] : a[k];
+                a[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < REST; k++)
+#pragma unroll
+            for (int o = LANES / 2; o >= 1; o >>= 1) a[MAIN + k] += __shfl_xor_sync(0xffffffffu, a[MAIN + k], o);
+        if (!store) return;
+#pragma unroll
+        for (int k = 0; k < (MAIN >> STEPS); k++)
+            if (base + k < COUNT - REST) row[base + k] = a[k];
+        if (l == 0)
+#pragma unroll
+            for (int k = 0; k < REST; k++) row[COUNT - REST + k] = a[MAIN + k];
+    }
+    __device__ __forceinline__ void load(const float *row) {
+        int n = 0;
+        each([&](float &v) { v = row[n++]; });
+    }
+};
+
+// one neighbour: X points at its interleaved V, A, B, R, C records
+template <bool CSPM, int COND>
+__device__ __forceinline__ void pair_body(const PairConst &P, const Target &I, const float4 Pj, const float4 *X,
+                                          Sums<CSPM, COND> &S) {
+    const float4 Vj = X[REC_V - 1], Aj = X[REC_A - 1], Bj = X[REC_B - 1], Cj = X[REC_C - 1];
+    const float2 nd = add2(lo2(Pj), I.nxy);  // -(x_i - x_j) in x, y
+    const float ndz = Pj.z + I.nz;
+    const float r2 = fmaf(ndz, ndz, fmaf(nd.y, nd.y, nd.x * nd.x));
+    const float rinv = rsqrt_approx(r2);  // r2 >= 1e-8 here: never a denormal
+    const float q = r2 * rinv * I.h1;
+    const float2 tu = make_float2(2.f - q, fmaxf(1.f - q, 0.f));
+    const float2 tu2 = mul2(tu, tu), tu3 = mul2(tu2, tu);
+    const float val = fmaf(0.25f, tu3.x, -tu3.y);
+    const float ng = fmaf(0.25f, tu2.x, -tu2.y) * rinv;  // -(u^2 - t^2/4)/r: g = ng * nd
+    const float2 g = mul2(both(ng), nd);
+    const float gz = ng * ndz;
+    const float vol = Cj.w;
+    if (!(I.tool == 1.f) && !(Pj.w == 1.f)) {
+        const float2 dv = add2(lo2(Vj), I.nvxy);         // v_j - v_i
+        const float2 zr = add2(hi2(Vj), I.nvz_rho);      // the z component; rho_i + rho_j
+        const float2 gx2 = both(g.x), gy2 = both(g.y), gz2 = both(gz);
+        {
+            const float2 a = mul2(both(vol), dv);
+            const float az = vol * zr.x;
+            S.Lx = fma2(a, gx2, S.Lx);
+            S.Ly = fma2(a, gy2, S.Ly);
+            S.Lz = fma2(a, gz2, S.Lz);
+            S.Lw = fma2(both(az), g, S.Lw);
+            S.Lzz = fmaf(az, gz, S.Lzz);
+        }
         // sum_j (sigma_i + sigma_j + fab (R_i + R_j)) g
-        //   = sum_j (sigma_j + fab R_j) g + sigma_i sum_j g + R_i sum_j fab g:
-        // slots 19-21 and 22-24 hold sum_j g and sum_j fab g, which the caller
-        // multiplies by the target's sigma and R once
-        float txx = Aj.x, tyy = Aj.y, tzz = Aj.z, txy = Aj.w, txz = Bj.x, tyz = Bj.y;
-        if (P.art) {
-            float fab = w * P.inv_wdeltap;
+        //   = sum_j (sigma_j + fab R_j) g + sigma_i sum_j g + R_i sum_j fab g
+        float2 t0 = lo2(Aj), t1 = hi2(Aj), t2 = lo2(Bj);  // (xx, xy), (xz, yz), (yy, zz)
+        if (I.art) {
+            const float4 Rj = X[REC_R - 1];
+            float fab = val * I.c_art;
             fab *= fab;
             fab *= fab;
-            txx = fmaf(fab, Rj.x, txx); tyy = fmaf(fab, Rj.y, tyy); tzz = fmaf(fab, Rj.z, tzz);
-            txy = fmaf(fab, Rj.w, txy); txz = fmaf(fab, Cj.x, txz); tyz = fmaf(fab, Cj.y, tyz);
-            acc[22] = fmaf(fab, gx, acc[22]); acc[23] = fmaf(fab, gy, acc[23]); acc[24] = fmaf(fab, gz, acc[24]);
+            const float2 fab2 = both(fab);
+            t0 = fma2(fab2, lo2(Rj), t0);
+            t1 = fma2(fab2, hi2(Rj), t1);
+            t2 = fma2(fab2, lo2(Cj), t2);
+            S.f = fma2(fab2, g, S.f);
+            S.fz = fmaf(fab, gz, S.fz);
         }
-        acc[19] += gx; acc[20] += gy; acc[21] += gz;
-        acc[9] = fmaf(txx, gx, fmaf(txy, gy, fmaf(txz, gz, acc[9])));
-        acc[10] = fmaf(txy, gx, fmaf(tyy, gy, fmaf(tyz, gz, acc[10])));
-        acc[11] = fmaf(txz, gx, fmaf(tyz, gy, fmaf(tzz, gz, acc[11])));
-        const float vr = -(dvx * dx + dvy * dy + dvz * dz);  // (v_i - v_j).(x_i - x_j)
-        const float rhoij = 0.5f * (I.rho + Vj.w);
-        const float irho = __fdividef(1.0f, rhoij);
-        {   // artificial viscosity for approaching pairs (vr < 0), without a branch
-            const float cij = 0.5f * (I.c + Bj.z), hij = 0.5f * (I.h + Bj.w);
-            const float mu = vr < 0.f ? __fdividef(hij * vr, r2 + P.eta2 * hij * hij) : 0.f;
-            const float pij = (-P.alpha * cij * mu + P.beta * mu * mu) * irho;
-            acc[12] = fmaf(-pij, gx, acc[12]);
-            acc[13] = fmaf(-pij, gy, acc[13]);
-            acc[14] = fmaf(-pij, gz, acc[14]);
+        S.g = add2(S.g, g);
+        S.gz += gz;
+        if (CSPM) {
+            S.s0[0] = fma2(t0, gx2, S.s0[0]); S.s0[1] = fma2(t0, gy2, S.s0[1]); S.s0[2] = fma2(t0, gz2, S.s0[2]);
+            S.s1[0] = fma2(t1, gx2, S.s1[0]); S.s1[1] = fma2(t1, gy2, S.s1[1]); S.s1[2] = fma2(t1, gz2, S.s1[2]);
+            S.s2[0] = fma2(t2, gx2, S.s2[0]); S.s2[1] = fma2(t2, gy2, S.s2[1]); S.s2[2] = fma2(t2, gz2, S.s2[2]);
+            // B = -sum V_j d (x) grad W with d = -nd
+            const float2 w = mul2(both(vol), nd);
+            S.b0 = fma2(both(w.x), g, S.b0);
+            S.b1 = fma2(both(w.y), make_float2(g.y, gz), S.b1);
+            S.bxz = fmaf(w.x, gz, S.bxz);
+            S.bzz = fmaf(vol * ndz, gz, S.bzz);
+        } else {
+            S.dx2 = fma2(t0, g, S.dx2);
+            S.dz2 = fma2(t1, g, S.dz2);
+            S.dxy = fma2(t1, gz2, S.dxy);
+            S.dy = fmaf(t0.y, g.x, fmaf(t2.x, g.y, S.dy));
+            S.dz = fmaf(t2.y, gz, S.dz);
         }
-        const float xw = w * irho;
-        acc[15] = fmaf(-xw, dvx, acc[15]);  // (w/rho_ij)(v_i - v_j)
-        acc[16] = fmaf(-xw, dvy, acc[16]);
-        acc[17] = fmaf(-xw, dvz, acc[17]);
+        const float ir = rcp_approx(zr.y);  // 1 / (rho_i + rho_j)
+        {   // artificial viscosity for approaching pairs, without a branch:
+            // mu = h_ij v.r/(r2 + eta^2 h_ij^2), h_ij = hs/2 (m = 2 mu), c_ij = cs/2
+            const float2 cs = add2(hi2(Bj), I.ch);
+            const float vr = fminf(fmaf(zr.x, ndz, fmaf(dv.y, nd.y, dv.x * nd.x)), 0.f);
+            const float m = vr * cs.y * rcp_approx(fmaf(P.eta2_4 * cs.y, cs.y, r2));
+            const float npij = -m * fmaf(P.beta_2, m, P.alpha_2 * cs.x) * ir;
+            S.av = fma2(both(npij), g, S.av);
+            S.avz = fmaf(npij, gz, S.avz);
+        }
+        const float xw = val * ir;
+        S.xs = fma2(both(xw), dv, S.xs);
+        S.xsz = fmaf(xw, zr.x, S.xsz);
     }
     if (COND == MFREE_COND_BROOKSHAW) {
-        // 2 (m/rho_j)(T_i - T_j) e.grad W / r = 2 V_j (T_i - T_j) (d.grad W)/r^2; factor 2 in the epilogue
-        acc[18] = fmaf(volj * (I.T - Cj.z), __fdividef(dx * gx + dy * gy + dz * gz, r2), acc[18]);
+        // 2 (m/rho_j)(T_i - T_j) e.grad W / r = 2 V_j (T_i - T_j) (d.grad W)/r^2; factor 2 in the
+        // epilogue.  Without CSPM d.g/r^2 is the pair's factor -ng.
+        const float k = -vol * (I.T - Cj.z) * ng;
+        if (CSPM) {
+            const float w = k * rinv * rinv;
+            const float2 v = mul2(both(w), nd);
+            S.h0 = fma2(both(v.x), nd, S.h0);
+            S.h1 = fma2(both(v.y), make_float2(nd.y, ndz), S.h1);
+            S.hxz = fmaf(v.x, ndz, S.hxz);
+            S.hzz = fmaf(w * ndz, ndz, S.hzz);
+        } else {
+            S.heat += k;
+        }
+    }
+}
+
+// the target's values from its records (h1, c_art and art are set apart)
+template <bool CSPM, int COND> __device__ __forceinline__ void target_of(const float4 Pi, const float4 *X, Target &I) {
+    const float4 Vi = X[REC_V - 1];
+    I.nxy = make_float2(-Pi.x, -Pi.y);
+    I.nz = -Pi.z;
+    I.tool = Pi.w;
+    I.nvxy = make_float2(-Vi.x, -Vi.y);
+    I.nvz_rho = make_float2(-Vi.z, Vi.w);
+    I.ch = hi2(X[REC_B - 1]);
+    I.T = X[REC_C - 1].z;
+}
+
+// the joined sums as the epilogue takes them: 0-8 velocity gradient, 9-11
+// stress divergence, 12-14 viscosity, 15-17 XSPH, 18 heat (Brookshaw)
+template <bool CSPM, int COND>
+__device__ __forceinline__ void finish_sums(const Sums<CSPM, COND> &S, const Target &I, float fac, const float4 Ai,
+                                            const float4 Bi, const float4 Ri, const float4 Ci, float *o) {
+    const float sc = 3.f * fac * I.h1;  // grad W = sc g
+    // rows of the correction (times sc); the identity without CSPM
+    float M[6] = {sc, sc, sc, 0.f, 0.f, 0.f};  // xx, yy, zz, xy, xz, yz
+    if (CSPM) {
+        float B[6] = {sc * S.b0.x, sc * S.b1.x, sc * S.bzz, sc * S.b0.y, sc * S.bxz, sc * S.b1.y}, inv[6];
+        const float det = det3s(B);
+        if (det > 9.99999994e-9f) {
+            inv3s(B, det, inv);
+#pragma unroll
+            for (int k = 0; k < 6; k++) M[k] = sc * inv[k];
+        }
+    }
+    auto corr = [&](float gx, float gy, float gz, float &x, float &y, float &z) {
+        if (CSPM) {
+            x = fmaf(M[0], gx, fmaf(M[3], gy, M[4] * gz));
+            y = fmaf(M[3], gx, fmaf(M[1], gy, M[5] * gz));
+            z = fmaf(M[4], gx, fmaf(M[5], gy, M[2] * gz));
+        } else {
+            x = sc * gx; y = sc * gy; z = sc * gz;
+        }
+    };
+    corr(S.Lx.x, S.Ly.x, S.Lz.x, o[0], o[1], o[2]);
+    corr(S.Lx.y, S.Ly.y, S.Lz.y, o[3], o[4], o[5]);
+    corr(S.Lw.x, S.Lw.y, S.Lzz, o[6], o[7], o[8]);
+    if (CSPM) {
+        float a, b, c, x, y, z;
+        corr(S.s0[0].x, S.s0[1].x, S.s0[2].x, x, y, z);  // t_xx
+        a = x;
+        corr(S.s0[0].y, S.s0[1].y, S.s0[2].y, x, y, z);  // t_xy
+        a += y; b = x;
+        corr(S.s1[0].x, S.s1[1].x, S.s1[2].x, x, y, z);  // t_xz
+        a += z; c = x;
+        corr(S.s1[0].y, S.s1[1].y, S.s1[2].y, x, y, z);  // t_yz
+        b += z; c += y;
+        corr(S.s2[0].x, S.s2[1].x, S.s2[2].x, x, y, z);  // t_yy
+        b += y;
+        corr(S.s2[0].y, S.s2[1].y, S.s2[2].y, x, y, z);  // t_zz
+        c += z;
+        o[9] = a; o[10] = b; o[11] = c;
+    } else {
+        o[9] = sc * S.dx2.x;
+        o[10] = sc * S.dy;
+        o[11] = sc * S.dz;
+    }
+    float gx, gy, gz, fx, fy, fz;
+    corr(S.g.x, S.g.y, S.gz, gx, gy, gz);
+    corr(S.f.x, S.f.y, S.fz, fx, fy, fz);
+    // sigma_i sum g + R_i sum fab g; A = (xx, xy, xz, yz), B = (yy, zz, ..), R, C alike
+    o[9] = fmaf(Ai.x, gx, fmaf(Ai.y, gy, fmaf(Ai.z, gz, o[9])));
+    o[10] = fmaf(Ai.y, gx, fmaf(Bi.x, gy, fmaf(Ai.w, gz, o[10])));
+    o[11] = fmaf(Ai.z, gx, fmaf(Ai.w, gy, fmaf(Bi.y, gz, o[11])));
+    o[9] = fmaf(Ri.x, fx, fmaf(Ri.y, fy, fmaf(Ri.z, fz, o[9])));
+    o[10] = fmaf(Ri.y, fx, fmaf(Ci.x, fy, fmaf(Ri.w, fz, o[10])));
+    o[11] = fmaf(Ri.z, fx, fmaf(Ri.w, fy, fmaf(Ci.y, fz, o[11])));
+    corr(S.av.x, S.av.y, S.avz, o[12], o[13], o[14]);
+    const float xf = -2.f * fac;  // W/rho_ij (v_i - v_j) = -2 fac val/(rho_i + rho_j) dv
+    o[15] = xf * S.xs.x; o[16] = xf * S.xs.y; o[17] = xf * S.xsz;
+    if (COND == MFREE_COND_BROOKSHAW) {
+        if (CSPM)
+            o[18] = M[0] * S.h0.x + M[1] * S.h1.x + M[2] * S.hzz + 2.f * (M[3] * S.h0.y + M[4] * S.hxz + M[5] * S.h1.y);
+        else
+            o[18] = sc * S.heat;
     }
 }
 
@@ -301,9 +555,9 @@ __device__ void epilogue(const StepArgs &a, int i, const float *res) {
 }
 
 // ---------------------------------------------------------- pair kernel --
-// Tile = TX x TY x TZ cells of the cell grid; its particles are 16 contiguous
+// Tile = TX x TY x D cells of the cell grid; its particles are 16 contiguous
 // column ranges of the sorted order.  Their 5x5x5 stencils lie in the halo of
-// HX x HY x HZ cells: 64 contiguous column ranges of the P records and of the
+// HX x HY x (D+4) cells: 64 contiguous column ranges of the P records and of the
 // interleaved rest, which two bulk copies per column (cp.async.bulk,
 // completion counted on an mbarrier) stage into shared memory in the same
 // layout.  A tile whose halo exceeds the staging capacity reads the same
@@ -312,72 +566,45 @@ constexpr int HX = TX + 4, HY = TY + 4;
 constexpr int CSROW = TILE_Z_MAX + 5;  // cell starts kept per halo column
 constexpr int NHC = HX * HY;           // halo columns
 constexpr int NTC = TX * TY;           // target columns
-// threads per block: 640 (20 warps, 96 registers a thread, a few spilled)
-// beat 512 (16 warps, 128 registers) by about 2 % on the 1M-particle scene
-// (CSPM + PSE) and by about 1 % on the mixed-size scenes (Brookshaw); 672 and
-// more threads leave at most 80 registers a thread, and the spills win
-template <bool CSPM> __host__ __device__ constexpr int tile_threads() { return 640; }
-constexpr int TCAP = 320;              // targets per pass of a tile
-constexpr int QCAP_T = 96;             // in-support queue per target before the rescan path
+constexpr int LPT = 2;                 // lanes per target
+constexpr int NCOMP = 480;             // compute threads
+constexpr int NTHREADS = NCOMP + 32;   // and the producer warp: 16 warps, 128 registers a thread
+constexpr int TCAP = NCOMP / LPT;      // targets per pass of a tile
+constexpr int QCAP = 96;               // in-support queue per target before the rescan path
+constexpr int CH = 4;                  // candidates a lane tests at once
+constexpr int QROW = 102;              // 204 bytes a target: the rows of a warp on different banks, and room for its sums
 
-// The in-support queue and the column walk of a group.  A staged tile's
-// record indices are below the staging capacity, so its queue entries are 16
-// bits and a column-walk entry packs the column's end in the flattened order
-// (low 16 bits) with the record-minus-flattened index offset (high 16 bits,
-// signed): both lie within the capacity.  A tile read from global memory keeps
-// 32-bit entries, placed in the staging area that such a tile leaves idle.
-template <bool STAGED> struct Walk {
-    using Q = unsigned short;
-    using C = int;
-    static __device__ __forceinline__ C pack(int end, int off) { return int(unsigned(off) << 16) | end; }
-    static __device__ __forceinline__ int end(C w) { return w & 0xffff; }
-    static __device__ __forceinline__ int off(C w) { return w >> 16; }
-};
-template <> struct Walk<false> {
-    using Q = int;
-    using C = int2;
-    static __device__ __forceinline__ C pack(int end, int off) { return make_int2(end, off); }
-    static __device__ __forceinline__ int end(C w) { return w.x; }
-    static __device__ __forceinline__ int off(C w) { return w.y; }
-};
 constexpr int SMEM_LIMIT = 232448;     // per-block shared memory of sm_100
 constexpr long long WAIT_CYCLES = 1ll << 30;  // bound of a staging wait (~0.5 s of SM clock)
 
-template <int LPP, int TILE_WARPS> struct TileSmem {
-    static constexpr int G = 32 / LPP;
-    float res[TCAP][NRES + 1];
-    int tgt[TCAP];       // sorted index of each target of the pass
-    int tcell[TCAP];     // its cell: target column << 16 | z
-    unsigned short q[TILE_WARPS][G][QCAP_T];
-    // per stencil column of a group's target: end of its candidates in the
-    // flattened order and record index minus flattened index (Walk<true>)
-    int cwalk[TILE_WARPS][G][25];
-    int cellstart[NHC][CSROW];
-    int hoff[NHC];       // staged offset of a halo column
-    int hstart[NHC];     // global start of a halo column
-    int hlen[NHC];
-    int tstart[NTC];
-    int tpref[NTC + 1];
+// a tile's tables, built by the producer warp one tile ahead (two buffers)
+struct TileTab {
+    int cs[NHC][CSROW];   // record index (staged) or sorted index of the cell starts of each halo column
+    int trec[NTC];        // record index of each target column's first target
+    int tsrt[NTC];        // its sorted index
+    int tpref[NTC + 1];   // targets before the column
+    float4 org;           // stencil pruning: grid origin, w = margin in cells (0: off)
+    int tile, depth, scene, args, total, staged;  // scene < 0: no tile left; args: slot of the scene's arguments
+    int nzr, rec0;        // cell starts in use per halo column; a target's record
+};
+struct BlockSmem {
+    TileTab tab[2];
     unsigned long long bar;
-    float4 org;        // stencil pruning of the current tile's scene: grid origin, 1 = on (no PSE only)
-    int tile, total, staged, parity, scene;  // scene < 0: no tile left
-    int next_args;     // scene whose arguments the second args buffer holds (-1: none)
-    int ntile, nscene; // the prologue threads' candidate tile
-    int2 pre_entry;    // tile-list entry fetched ahead for the next prologue
-    int pre_ok;        // pre_entry is being fetched (cp.async)
-    int list_n;        // entries of the tile list
+    int fail, list_n;
 };
 __host__ __device__ constexpr size_t round128(size_t b) { return (b + 127) / 128 * 128; }
-// shared memory: the tables, the scene's arguments, the staged records
-template <int LPP, int W> __host__ __device__ constexpr size_t args_offset() {
-    return round128(sizeof(TileSmem<LPP, W>));
-}
-template <int LPP, int W> __host__ __device__ constexpr size_t rec_offset() {
-    return args_offset<LPP, W>() + 2 * round128(sizeof(StepArgs));  // the current and the next tile's scene
-}
-template <int LPP, int W> __host__ __device__ constexpr int rec_capacity() {
-    return int((SMEM_LIMIT - rec_offset<LPP, W>()) / (REC_N * sizeof(float4)));
-}
+// shared memory: the tables, the arguments of two scenes, the queues, the staged records
+constexpr size_t ARGS_OFFSET = round128(sizeof(BlockSmem));
+constexpr size_t ARGS_SIZE = round128(sizeof(StepArgs));
+constexpr size_t QUEUE_OFFSET = ARGS_OFFSET + 2 * ARGS_SIZE;
+constexpr size_t REC_OFFSET = round128(QUEUE_OFFSET + size_t(TCAP) * QROW * sizeof(unsigned short));
+constexpr int REC_CAP = int((SMEM_LIMIT - REC_OFFSET) / (REC_N * sizeof(float4)));
+// a tile read from global memory keeps 32-bit queue entries in the idle staging area
+static_assert(size_t(TCAP) * QROW * sizeof(int) <= size_t(REC_CAP) * REC_N * sizeof(float4), "queue in the staging area");
+static_assert(CH * LPT <= REC_CAP, "reads past a column stay in the staging area");
+static_assert(QROW * sizeof(unsigned short) >= 51 * sizeof(float) && QROW >= QCAP, "a target's sums fit its queue row");
+static_assert(TILE_HALO_MAX + NHC <= REC_CAP, "the estimated halo and its parity gaps fit the staging area");
+static_assert(REC_CAP < 65536, "16-bit queue entries");
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return unsigned(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(unsigned long long *b, unsigned n) {
@@ -402,719 +629,535 @@ __device__ __forceinline__ void bulk_to_smem(void *dst, const void *src, unsigne
                  : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Named barriers, each passed once per tile (a warp that waits at one takes no
+// issue slots; fifteen warps polling the mbarrier took a third of them):
+//   BAR_FULL   everybody: the tile's records have landed and its tables are
+//              built, and the compute warps are done with the tile before
+//   BAR_READ   the compute warps (which only arrive) have read their last
+//              record of the tile; the producer waits for it
+// and one among the compute warps alone, with an AND of a predicate.
+constexpr int BAR_FULL = 1, BAR_READ = 2, BAR_COMPUTE = 3;
+// (the aligned forms: a warp's lanes arrive together)
+template <int ID> __device__ __forceinline__ void bar_arrive() {
+    __syncwarp();
+    asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(NTHREADS) : "memory");
+}
+template <int ID> __device__ __forceinline__ void bar_wait() {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(NTHREADS) : "memory");
+}
+__device__ __forceinline__ bool compute_and(bool v) {
+    unsigned r;
+    __syncwarp();
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(r)
+                 : "r"(unsigned(v)), "n"(BAR_COMPUTE), "n"(NCOMP)
+                 : "memory");
+    return r != 0;
+}
 
-// inclusive scan over the LPP lanes of a group
-template <int LPP> __device__ __forceinline__ int group_scan(int v, int sl) {
+__device__ __forceinline__ int warp_scan(int v, int lane) {
 #pragma unroll
-    for (int o = 1; o < LPP; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, v, o, LPP);
-        if (sl >= o) v += y;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
     }
     return v;
 }
 
-// the records of one kind at a fixed stride: P alone, the other five
-// interleaved per particle
-template <int S> struct RecView {
-    const float4 *__restrict__ p;
-    __device__ __forceinline__ const float4 &operator[](int j) const { return p[j * S]; }
-};
-
-// one target: stencil ranges, pass A (support, PSE, queue), CSPM pass over
-// the queue, pair pass over the queue, group reduction
-template <int LPP, bool CSPM, int COND, bool STAGED, class SM>
-__device__ __forceinline__ void process_target(const StepArgs &a, SM &sm, float4 *spare, const float4 *RF, int rstride,
-                                               int i, bool valid, int tt, int warp, int g, int sl, int lane, int X0,
-                                               int Y0, int zl) {
+// One pass over the targets of a tile: lane pair (tt, sl) serves target tt
+// from its candidates to its reduced sums.  Returns the target's sorted index
+// (-1: none) and its results in res[0..19] (19: neighbours in support).
+template <bool CSPM, int COND, bool STAGED>
+__device__ __forceinline__ int process_target(const StepArgs &a, const TileTab &tab, unsigned short *queue,
+                                              float4 *sarr, int ntg, int tt, int sl, int rounds, float *res) {
     const Params &P = a.p;
-    const int nx = P.gnx, ny = P.gny, nz = P.gnz;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const unsigned gmask = LPP == 32 ? 0xffffffffu : (((1u << LPP) - 1u) << (g * LPP));
-    // the records of rstride particles (shared memory or global): P at RF,
-    // V, A, B, R, C interleaved from RF + rstride
-    const float4 *X = RF + rstride;
-    const RecView<1> rP{RF};
-    const RecView<REC_X> rV{X + (REC_V - 1)}, rA{X + (REC_A - 1)}, rB{X + (REC_B - 1)}, rR{X + (REC_R - 1)},
-        rC{X + (REC_C - 1)};
-    // the target's cell (from the pass's target table); its own records come
-    // from the staged halo (its cell column is one of the halo's) or from
-    // global memory
-    const int tcell = sm.tcell[valid ? tt : 0];
-    const int gi = X0 + (tcell >> 16) / TY, gj = Y0 + (tcell >> 16) % TY, gk = tcell & 0xffff;
-    IData I;
-    int si = i;  // the target's own record
-    if (STAGED) {
-        const int lc = (gi - X0 + 2) * HY + (gj - Y0 + 2);
-        si = sm.hoff[lc] + (i - sm.hstart[lc]);
-        if (!bounds_ok(a.clk, si, rstride)) si = 0;
+    using Q = typename std::conditional<STAGED, unsigned short, int>::type;
+    // the records: P at RF, V, A, B, R, C interleaved from RF + rn
+    const float4 *__restrict__ RF = STAGED ? sarr : a.r.f[REC_P];
+    const int rn = STAGED ? REC_CAP : P.n_init;
+    const float4 *__restrict__ X = RF + rn;
+    const bool valid = tt < ntg;
+    const TileGeo G = tile_geo(P, tab.tile, tab.depth);
+    // the target: its column, sorted index, record and cell
+    int i = -1, si = 0, c = 0, gk = G.Z0;
+    if (valid) {
+#pragma unroll
+        for (int k = NTC / 2; k >= 1; k >>= 1)
+            if (tab.tpref[c + k] <= tt) c += k;
+        i = tab.tsrt[c] + (tt - tab.tpref[c]);
+        si = tab.trec[c] + (tt - tab.tpref[c]);
+        if (!bounds_ok(a.clk, i, P.n_init)) i = 0;
+        if (!bounds_ok(a.clk, si, rn)) si = 0;
+        const int *cs = tab.cs[(c / TY + 2) * HY + (c % TY + 2)];
+        int k = G.Z0 - G.zl;
+        while (k < G.nzr - 2 && cs[k + 1] <= si) k++;
+        gk = G.zl + k;
     }
+    Target I;
+    float h, fac;
     {
-        const float4 Pi = rP[si], Vi = rV[si], Bi = rB[si], Ci = rC[si];
-        I.x = Pi.x; I.y = Pi.y; I.z = Pi.z; I.tool = Pi.w;
-        I.vx = Vi.x; I.vy = Vi.y; I.vz = Vi.z; I.rho = Vi.w;
-        I.c = Bi.z; I.h = Bi.w;
-        I.T = Ci.z;
-        I.h1 = 1.0f / I.h;
-        I.fac = 0.31830988618379067f * I.h1 * I.h1 * I.h1;
+        target_of<CSPM, COND>(RF[si], X + si * REC_X, I);
+        h = I.ch.y;
+        I.h1 = 1.0f / h;
+        fac = 0.31830988618379067f * I.h1 * I.h1 * I.h1;
+        I.art = P.wdeltap > 0.f;
+        I.c_art = fac * P.inv_wdeltap;
     }
-    using WK = Walk<STAGED>;
-    typename WK::C *cw;
-    typename WK::Q *qq;
-    if (STAGED) {
-        cw = reinterpret_cast<typename WK::C *>(sm.cwalk[warp][g]);
-        qq = reinterpret_cast<typename WK::Q *>(sm.q[warp][g]);
-    } else {  // 32-bit entries in the idle staging area
-        constexpr int NG = int(sizeof(sm.q) / sizeof(sm.q[0][0]));  // groups of the block
-        int *q32 = reinterpret_cast<int *>(spare);
-        qq = reinterpret_cast<typename WK::Q *>(q32 + (warp * SM::G + g) * QCAP_T);
-        cw = reinterpret_cast<typename WK::C *>(reinterpret_cast<int2 *>(q32 + NG * QCAP_T) + (warp * SM::G + g) * 25);
-    }
-    int total;  // candidates of the target
-    // ---- the 25 stencil columns as ranges of the record arrays, with their
-    // prefix.  Without PSE (which sums every candidate of the 5x5x5 cells) the
+    // ---- the candidates: lane sl takes the records of parity sl of each
+    // stencil column.  Without PSE (which sums every candidate of the 5x5x5 cells) the
     // cells that lie wholly beyond the target's support radius are left out
     // (org.w = the margin in cells, 0 = off; org.xyz = the grid origin of this
     // step's hash): in cell units, a column's x-y box and a cell's z extent,
     // each widened by the margin, against the sphere of radius 2h around the
-    // target.  Only
-    // out-of-support candidates go, in the same order, so the in-support
+    // target.  Only out-of-support candidates go, in the same order, so the
     // queue and every sum over it are unchanged.  Cell 0 of an axis also holds
     // positions up to one cell below the origin (the hash truncates toward 0).
     constexpr bool PRUNE = COND != MFREE_COND_PSE;
-    const float4 org = PRUNE ? sm.org : make_float4(0.f, 0.f, 0.f, 0.f);
-    float ux = 0.f, uy = 0.f, uz = 0.f, rc2 = 0.f;
-    if (PRUNE && org.w != 0.f) {
-        const float ic = 1.0f / P.gdx;
-        ux = (I.x - org.x) * ic;
-        uy = (I.y - org.y) * ic;
-        uz = (I.z - org.z) * ic;
-        const float rc = 2.0f * I.h * ic;
-        rc2 = rc * rc;
-    }
-    {
-        const int klo = max(gk - 2, 0), khi = min(gk + 2, nz - 1);
-        constexpr int NSET = (25 + LPP - 1) / LPP;
-        int carry = 0;
-#pragma unroll
-        for (int k = 0; k < NSET; k++) {
-            const int c = sl + k * LPP;
-            int b = 0, l = 0;
-            if (valid && c < 25) {
-                const int cx = gi + c / 5 - 2, cy = gj + c % 5 - 2;
-                if (cx >= 0 && cx < nx && cy >= 0 && cy < ny) {
-                    int k0 = klo, k1 = khi;
-                    if (PRUNE && org.w != 0.f) {
-                        const float mg = org.w;
-                        const float lox = (cx == 0 ? -1.f : float(cx)) - mg;
-                        const float loy = (cy == 0 ? -1.f : float(cy)) - mg;
-                        const float ex = fmaxf(0.f, fmaxf(lox - ux, ux - (float(cx + 1) + mg)));
-                        const float ey = fmaxf(0.f, fmaxf(loy - uy, uy - (float(cy + 1) + mg)));
-                        const float d2 = ex * ex + ey * ey;
-                        if (d2 < rc2) {
-                            const float zr = sqrtf(rc2 - d2) + mg;
-                            int z1 = int(floorf(uz + zr));
-                            if (z1 < 0 && uz + zr > -1.f) z1 = 0;
-                            k0 = max(k0, int(floorf(uz - zr)));
-                            k1 = min(k1, z1);
-                        } else {
-                            k1 = k0 - 1;
-                        }
-                    }
-                    if (k1 >= k0) {
-                        const int lc = (cx - X0 + 2) * HY + (cy - Y0 + 2);
-                        const int s0 = sm.cellstart[lc][k0 - zl];
-                        l = sm.cellstart[lc][k1 + 1 - zl] - s0;
-                        b = STAGED ? sm.hoff[lc] + (s0 - sm.hstart[lc]) : s0;
-                    }
-                }
-            }
-            const int inc = group_scan<LPP>(l, sl);
-            if (c < 25) cw[c] = WK::pack(carry + inc, b - (carry + inc - l));
-            carry += __shfl_sync(0xffffffffu, inc, (g * LPP) + LPP - 1);
-        }
-        total = carry;
-    }
-    __syncwarp();
-    // ---- candidates: lane sl takes candidates sl, sl + LPP, ... of the
-    // flattened stencil (consecutive lanes read consecutive records); the
-    // column it is in is kept in registers and reloaded only on a crossing
-    int maxtotal = total;
-#pragma unroll
-    for (int o = 16; o >= LPP; o >>= 1) maxtotal = max(maxtotal, __shfl_xor_sync(0xffffffffu, maxtotal, o));
+    const float4 org = tab.org;
+    const bool prune = PRUNE && org.w != 0.f;
+    const int klo = max(gk - 2, 0), khi = min(gk + 2, P.gnz - 1);
+    const int *cs0 = tab.cs[(c / TY) * HY + (c % TY)];  // the stencil's first column
     auto scan = [&](auto &&fn) {
-        int col = 0;
-        typename WK::C w = cw[0];
-        int cend = WK::end(w), base = WK::off(w);
-#pragma unroll 2
-        for (int k0 = 0; k0 < maxtotal; k0 += LPP) {
-            const int k = k0 + sl;
-            const bool act = k < total;
-            if (act) {
-                while (k >= cend) {  // k < total keeps col <= 24
-                    col++;
-                    w = cw[col];
-                    cend = WK::end(w);
-                    base = WK::off(w);
+        if (!valid) return;
+        const int gi = G.X0 + c / TY, gj = G.Y0 + c % TY;
+        float ux = 0.f, uy = 0.f, uz = 0.f, rc2 = 0.f;
+        if (prune) {
+            const float ic = 1.0f / P.gdx;
+            ux = (-I.nxy.x - org.x) * ic;
+            uy = (-I.nxy.y - org.y) * ic;
+            uz = (-I.nz - org.z) * ic;
+            const float rc = 2.0f * h * ic;
+            rc2 = rc * rc;
+        }
+#pragma unroll 1
+        for (int ca = 0; ca < 5; ca++) {
+            const int cx = gi + ca - 2;
+            const float ex = fmaxf(0.f, fmaxf((cx == 0 ? -1.f : float(cx)) - org.w - ux, ux - (float(cx + 1) + org.w)));
+            const float rx2 = rc2 - ex * ex;
+            const int *row = cs0 + ca * (HY * CSROW) - G.zl;
+            // the record ranges of five columns at once: their latencies overlap
+            int js[5], je[5];
+#pragma unroll
+            for (int cb = 0; cb < 5; cb++) {
+                int k0 = klo, k1 = khi;
+                if (prune) {
+                    const int cy = gj + cb - 2;
+                    const float ey = fmaxf(0.f, fmaxf((cy == 0 ? -1.f : float(cy)) - org.w - uy, uy - (float(cy + 1) + org.w)));
+                    const float rz2 = rx2 - ey * ey;
+                    float z;
+                    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(z) : "f"(fmaxf(rz2, 0.f)));  // the margin covers its error
+                    const float zr = z + org.w;
+                    int z1 = __float2int_rd(uz + zr);
+                    if (z1 < 0 && uz + zr > -1.f) z1 = 0;
+                    k0 = max(k0, __float2int_rd(uz - zr));
+                    k1 = rz2 > 0.f ? min(k1, z1) : -1;
                 }
+                const bool some = k1 >= k0;
+                const int j0 = row[cb * CSROW + (some ? k0 : klo)], j1 = row[cb * CSROW + (some ? k1 : klo) + 1];
+                js[cb] = j0 + ((j0 ^ sl) & 1);
+                je[cb] = some ? j1 : 0;
             }
-            int j = base + k;
-            if (act && !bounds_ok(a.clk, j, rstride)) j = 0;
-            fn(j, act);
+#pragma unroll
+            for (int cb = 0; cb < 5; cb++) fn(js[cb], je[cb]);
         }
     };
-    // ---- pass A: support test, PSE, queue
+    // ---- support test, PSE, queue (filled by lane 0 from its start, by lane 1 from its end)
     const float pse_k = -1.44269504088896341f * I.h1 * I.h1;  // exp(-r^2/h^2) = 2^(pse_k r^2)
-    const float four_h2 = __fmul_rn(__fmul_rn(4.0f, I.h), I.h);
-    int qn = 0;  // in-support neighbours of the target (the group's ballots: the same in every lane)
+    const float four_h2 = __fmul_rn(__fmul_rn(4.0f, h), h);
+    Q *const qrow = (STAGED ? reinterpret_cast<Q *>(queue) : reinterpret_cast<Q *>(sarr)) + (threadIdx.x / LPT) * QROW;
+    Q *qp = sl == 0 ? qrow : qrow + (QCAP - 1);
+    const int qstep = sl == 0 ? 1 : -1;
+    int qn = 0;
     float pse = 0.f;
-    {   // two candidates per lane and iteration (k and k + LPP): both column
-        // walks, then both loads, then the arithmetic, so the shared-memory
-        // round trips overlap; the ballots keep the flattened order
-        int col = 0;
-        typename WK::C w = cw[0];
-        int cend = WK::end(w), base = WK::off(w);
-#pragma unroll 1
-        for (int k0 = 0; k0 < maxtotal; k0 += 2 * LPP) {
-            const int ka = k0 + sl, kb = ka + LPP;
-            const bool acta = ka < total, actb = kb < total;
-            int ja = 0, jb = 0;
-            if (acta) {
-                while (ka >= cend) {
-                    col++;
-                    w = cw[col];
-                    cend = WK::end(w);
-                    base = WK::off(w);
-                }
-                ja = base + ka;
-                if (!bounds_ok(a.clk, ja, rstride)) ja = 0;
-            }
-            if (actb) {
-                while (kb >= cend) {
-                    col++;
-                    w = cw[col];
-                    cend = WK::end(w);
-                    base = WK::off(w);
-                }
-                jb = base + kb;
-                if (!bounds_ok(a.clk, jb, rstride)) jb = 0;
-            }
-            float4 Pa = make_float4(0.f, 0.f, 0.f, 0.f), Pb = Pa;
-            float2 ta = make_float2(0.f, 0.f), tb = ta;
-            if (acta) {
-                Pa = rP[ja];
-                if (COND == MFREE_COND_PSE) ta = reinterpret_cast<const float2 *>(&rC[ja])[1];
-            }
-            if (actb) {
-                Pb = rP[jb];
-                if (COND == MFREE_COND_PSE) tb = reinterpret_cast<const float2 *>(&rC[jb])[1];
-            }
-            bool insa = false, insb = false;
-            if (acta) {
-                const float r2 = dist2_rn(I.x - Pa.x, I.y - Pa.y, I.z - Pa.z);
-                insa = !(r2 >= four_h2) && (r2 > 9.99999994e-9f);
-                if (COND == MFREE_COND_PSE) {
-                    float e2;
-                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e2) : "f"(pse_k * r2));
-                    pse = fmaf((ta.x - I.T) * ta.y, e2, pse);
-                }
-            }
-            if (actb) {
-                const float r2 = dist2_rn(I.x - Pb.x, I.y - Pb.y, I.z - Pb.z);
-                insb = !(r2 >= four_h2) && (r2 > 9.99999994e-9f);
-                if (COND == MFREE_COND_PSE) {
-                    float e2;
-                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e2) : "f"(pse_k * r2));
-                    pse = fmaf((tb.x - I.T) * tb.y, e2, pse);
-                }
-            }
-            const unsigned ma = __ballot_sync(0xffffffffu, insa) & gmask;
-            const unsigned mb = __ballot_sync(0xffffffffu, insb) & gmask;
-            const int qa = qn + __popc(ma & lt_mask), qb = qn + __popc(ma) + __popc(mb & lt_mask);
-            if (insa && qa < QCAP_T) qq[qa] = ja;
-            if (insb && qb < QCAP_T) qq[qb] = jb;
-            qn += __popc(ma) + __popc(mb);
-        }
-    }
-    if (COND == MFREE_COND_PSE) {  // the PSE sum waits in the target's result slot
-#pragma unroll
-        for (int o = LPP / 2; o >= 1; o >>= 1) pse += __shfl_xor_sync(0xffffffffu, pse, o);
-        if (sl == 0 && valid) sm.res[tt][18] = pse;
-    }
-    __syncwarp();
-    const int qv = min(qn, QCAP_T);
-    int maxq = qv;
-#pragma unroll
-    for (int o = 16; o >= LPP; o >>= 1) maxq = max(maxq, __shfl_xor_sync(0xffffffffu, maxq, o));
-    const bool overflow = __any_sync(0xffffffffu, qn > QCAP_T);
-    // in-support neighbours beyond the queue: found again by the same scan
-    auto for_overflow = [&](auto &&fn) {
-        int ord = 0;
-        scan([&](int j, bool act) {
-            bool ins = false;
-            if (act && qn > QCAP_T) {
-                const float4 Pj = rP[j];
-                ins = in_support(dist2_rn(I.x - Pj.x, I.y - Pj.y, I.z - Pj.z), I.h);
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, ins) & gmask;
-            const int pos = ord + __popc(m & lt_mask);
-            if (ins && pos >= QCAP_T) fn(j);
-            ord += __popc(m);
-        });
+    // the in-support test of the reference's neighbour count: the unfused sum
+    // of squares, 1e-8 <= r^2 < 4 h^2
+    auto dist2 = [&](const float4 Pj) {
+        const float2 d = add2(lo2(Pj), I.nxy);
+        const float dz = Pj.z + I.nz;
+        const float2 m = mul2(d, d);
+        return __fadd_rn(__fadd_rn(m.x, m.y), __fmul_rn(dz, dz));
     };
-    // ---- CSPM matrix over the in-support neighbours (interactions_gpu.cu:227-295)
-    float invB[6] = {1.f, 1.f, 1.f, 0.f, 0.f, 0.f};
-    if (CSPM) {
-        float Bm[6];  // xx, yy, zz, xy, xz, yz
-#pragma unroll
-        for (int k = 0; k < 6; k++) Bm[k] = 0.f;
-        // one neighbour's term: B += sv d (x) d with sv = -V_j dfac
-        auto bvals = [&](const float4 Pj, float vj) {
-            if (I.tool == 1.f || Pj.w == 1.f) return;
-            const float dx = I.x - Pj.x, dy = I.y - Pj.y, dz = I.z - Pj.z;
-            float w, dfac;
-            spline(dist2_rn(dx, dy, dz), I.h1, I.fac, w, dfac);
-            const float sv = -vj * dfac;
-            const float tx = sv * dx, ty = sv * dy, tz = sv * dz;
-            Bm[0] = fmaf(tx, dx, Bm[0]);
-            Bm[1] = fmaf(ty, dy, Bm[1]);
-            Bm[2] = fmaf(tz, dz, Bm[2]);
-            Bm[3] = fmaf(tx, dy, Bm[3]);
-            Bm[4] = fmaf(tx, dz, Bm[4]);
-            Bm[5] = fmaf(ty, dz, Bm[5]);
-        };
-        auto bterm = [&](int j) { bvals(rP[j], rC[j].w); };
-        // two queue entries per lane and iteration (q and q + LPP): both loads
-        // before either term, so the shared-memory round trips overlap; each
-        // lane still adds its terms in queue order
+    scan([&](int j, int je) {
+        // CH candidates a lane at once, without a branch: records past the
+        // column's end are read (they lie inside the record arrays) and masked
 #pragma unroll 1
-        for (int q0 = 0; q0 < maxq; q0 += 2 * LPP) {
-            const int qa = q0 + sl, qb = qa + LPP;
-            const bool a = qa < qv, b = qb < qv;
-            const int ja = a ? qq[qa] : 0, jb = b ? qq[qb] : 0;
-            float4 Pa = make_float4(0.f, 0.f, 0.f, 0.f), Pb = Pa;
-            float va = 0.f, vb = 0.f;
-            if (a) { Pa = rP[ja]; va = rC[ja].w; }
-            if (b) { Pb = rP[jb]; vb = rC[jb].w; }
-            if (a) bvals(Pa, va);
-            if (b) bvals(Pb, vb);
+        for (; j < je; j += CH * LPT) {
+            if (!bounds_ok(a.clk, j, rn)) continue;
+            float4 p[CH];
+            float2 tv[CH];
+#pragma unroll
+            for (int k = 0; k < CH; k++) {
+                p[k] = RF[j + k * LPT];
+                if (COND == MFREE_COND_PSE) tv[k] = hi2(X[min(j + k * LPT, rn - 1) * REC_X + (REC_C - 1)]);
+            }
+            const bool room = qn <= QCAP - CH;
+#pragma unroll
+            for (int k = 0; k < CH; k++) {
+                const float r2 = dist2(p[k]);
+                const bool have = j + k * LPT < je;
+                if (COND == MFREE_COND_PSE) {
+                    float e;
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(pse_k * r2));
+                    const float v = fmaf((tv[k].x - I.T) * tv[k].y, e, pse);
+                    pse = have ? v : pse;
+                }
+                const bool in = have && !(r2 >= four_h2) && r2 > 9.99999994e-9f;
+                if (in && room) *qp = Q(j + k * LPT);
+                if (in) qp += qstep;
+                qn += in ? 1 : 0;
+            }
         }
-        if (overflow) for_overflow(bterm);
-#pragma unroll
-        for (int o = LPP / 2; o >= 1; o >>= 1)
-#pragma unroll
-            for (int k = 0; k < 6; k++) Bm[k] += __shfl_xor_sync(0xffffffffu, Bm[k], o);
-        const float det = det3s(Bm);
-        if (det > 9.99999994e-9f) inv3s(Bm, det, invB);
-    }
-    // ---- pair body over the in-support neighbours
-    float acc[25];
-#pragma unroll
-    for (int k = 0; k < 25; k++) acc[k] = 0.f;
-    const PairConst PC{P.inv_wdeltap, P.av_eta * P.av_eta, P.av_alpha, P.av_beta, P.wdeltap > 0.f};
-    auto pterm = [&](int j) { pair_body<CSPM, COND>(PC, I, invB, rP[j], rV[j], rA[j], rB[j], rR[j], rC[j], acc); };
-    for (int q0 = 0; q0 < maxq; q0 += LPP) {
-        const int q = q0 + sl;
-        if (q < qv) pterm(qq[q]);
-    }
-    if (overflow) for_overflow(pterm);
-    {   // the target's own sigma and R: sigma_i sum g + R_i sum fab g, in each lane
-        const float4 Ai = rA[si], Bi = rB[si], Ri = rR[si], Ci = rC[si];
-        acc[9] = fmaf(Ai.x, acc[19], fmaf(Ai.w, acc[20], fmaf(Bi.x, acc[21], acc[9])));
-        acc[10] = fmaf(Ai.w, acc[19], fmaf(Ai.y, acc[20], fmaf(Bi.y, acc[21], acc[10])));
-        acc[11] = fmaf(Bi.x, acc[19], fmaf(Bi.y, acc[20], fmaf(Ai.z, acc[21], acc[11])));
-        acc[9] = fmaf(Ri.x, acc[22], fmaf(Ri.w, acc[23], fmaf(Ci.x, acc[24], acc[9])));
-        acc[10] = fmaf(Ri.w, acc[22], fmaf(Ri.y, acc[23], fmaf(Ci.y, acc[24], acc[10])));
-        acc[11] = fmaf(Ci.x, acc[22], fmaf(Ci.y, acc[23], fmaf(Ri.z, acc[24], acc[11])));
-    }
-    constexpr int NACC = COND == MFREE_COND_PSE ? 18 : 19;  // (slot 18 holds the PSE sum already)
-#pragma unroll
-    for (int o = LPP / 2; o >= 1; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < NACC; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-    }
-    if (sl == 0 && valid) {
-        float *rs = sm.res[tt];
-#pragma unroll
-        for (int k = 0; k < NACC; k++) rs[k] = acc[k];
-        rs[19] = __int_as_float(qn);
+    });
+    __syncwarp();
+    const int qo = __shfl_xor_sync(0xffffffffu, qn, 1);  // the other lane's neighbours
+    const int nq = qn + qo;
+    const bool queued = nq <= QCAP && max(qn, qo) <= QCAP - CH;
+    if (COND == MFREE_COND_PSE) pse += __shfl_xor_sync(0xffffffffu, pse, 1);
+    // ---- pair body over the in-support neighbours: eight lanes a target, four
+    // targets of the warp at a time; lanes 0-3 take the queue's front part,
+    // lanes 4-7 its back part.  Their entries are mostly neighbouring records,
+    // which lie on different banks (with two lanes a target the sixteen targets
+    // of a warp read unrelated records: 12 wavefronts a load instead of ~5).
+    // A target's sums replace its queue row.
+    const int lane = threadIdx.x & 31;
+    const PairConst PC{0.25f * P.av_eta * P.av_eta, -0.5f * P.av_alpha, 0.5f * P.av_beta};
+    {
+        const int l = lane & 7, back = l >> 2;
+        Q *const wrow = qrow - size_t(lane / LPT) * QROW;  // the warp's first row
+#pragma unroll 1
+        for (int rd = 0; rd < rounds; rd++) {
+            const int tl = rd * 4 + (lane >> 3), own = tl * LPT;
+            const int n_f = __shfl_sync(0xffffffffu, queued && valid ? qn : 0, own);
+            const int n_b = __shfl_sync(0xffffffffu, queued && valid ? qn : 0, own + 1);
+            const int sj = __shfl_sync(0xffffffffu, si, own);
+            const unsigned busy = __ballot_sync(0xffffffffu, n_f + n_b > 0);
+            if (busy == 0) continue;
+            Target J;
+            J.h1 = __shfl_sync(0xffffffffu, I.h1, own);
+            J.c_art = __shfl_sync(0xffffffffu, I.c_art, own);
+            J.art = I.art;
+            target_of<CSPM, COND>(RF[sj], X + sj * REC_X, J);
+            Q *const row = wrow + tl * QROW;
+            const Q *qe = back ? row + (QCAP - 1) - (l & 3) : row + (l & 3);
+            const int qd = back ? -4 : 4, cnt = back ? n_b : n_f;
+            Sums<CSPM, COND> S;
+            S.zero();
+            // the next entry's index and position are read ahead
+            int m = l & 3;
+            int j = m < cnt ? int(*qe) : sj;
+            float4 Pj = RF[j];
+            int jn = m + 4 < cnt ? int(qe[qd]) : j;
+#pragma unroll 1
+            for (; m < cnt; m += 4) {
+                const float4 Pc = Pj;
+                const int jc = j;
+                j = jn;
+                Pj = RF[j];
+                qe += qd;
+                jn = m + 8 < cnt ? int(qe[qd]) : j;
+                pair_body<CSPM, COND>(PC, J, Pc, X + jc * REC_X, S);
+            }
+            __syncwarp();
+            S.template reduce_to<8>(reinterpret_cast<float *>(row), l, n_f + n_b > 0);
+        }
     }
     __syncwarp();
+    Sums<CSPM, COND> S;
+    S.zero();
+    float *const srow = reinterpret_cast<float *>(qrow);
+    if (__any_sync(0xffffffffu, !queued)) {  // queues that overflowed: the neighbours are found again by the same scan
+        if (!queued)
+            scan([&](int j, int je) {
+#pragma unroll 1
+                for (; j < je; j += LPT) {
+                    if (!bounds_ok(a.clk, j, rn)) continue;
+                    const float4 Pj = RF[j];
+                    const float r2 = dist2(Pj);
+                    if (!(r2 >= four_h2) && r2 > 9.99999994e-9f) pair_body<CSPM, COND>(PC, I, Pj, X + j * REC_X, S);
+                }
+            });
+        __syncwarp();
+        S.template reduce_to<LPT>(srow, sl, !queued);
+        __syncwarp();
+    }
+    if (nq > 0 && valid) S.load(srow);
+    const float4 Ai = X[si * REC_X + (REC_A - 1)], Bi = X[si * REC_X + (REC_B - 1)], Ri = X[si * REC_X + (REC_R - 1)],
+                 Ci = X[si * REC_X + (REC_C - 1)];
+    finish_sums<CSPM, COND>(S, I, fac, Ai, Bi, Ri, Ci, res);
+    if (COND == MFREE_COND_PSE) res[18] = pse;
+    if (COND == MFREE_COND_NONE) res[18] = 0.f;
+    res[19] = __int_as_float(nq);
+    return i;
 }
 
-// threads at or above PRO_FIRST never run the epilogue (TCAP <= PRO_FIRST):
-// while the others finish the current tile, they prepare the next one
-constexpr int PRO_FIRST = TCAP;
-__device__ __forceinline__ void pro_sync(int nthreads) { asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory"); }
-
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\ncp.async.commit_group;" ::"r"(smem_u32(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Run by the prologue threads: takes the next entry of the tile list (the
-// non-empty tiles of every scene), copies its scene's arguments into the
-// second args buffer when the scene is not the current tile's (busy_scene),
-// builds its halo cell starts, its target ranges (read from the halo table:
-// the target columns are halo columns) and halo offsets, and issues its
-// staging copies.  The prepared tile is left in sm.tile / sm.scene (scene < 0:
-// none left).  Once its copies are issued, each call claims the list entry of
-// the next call and starts fetching it into shared memory: the claim's round
-// trip then overlaps the copies, and neither it nor the entry's load waits in
-// the next call (a global atomic still in flight holds up the barrier that
-// follows it until it is performed).  The target table and the halo table are
-// built by two warps at once, the halo table with one scan (lane l owns halo
-// columns 2l and 2l + 1; the staged order of the columns is free).  The caller
-// guarantees that nothing reads the staged records or the tile tables any
-// more.  Kept out of line: inlined into the kernel's loop it made the pair
-// rounds about 7% slower (measured on the 1M-particle step).
-template <int LPP, int W, int CAP>
-__device__ __noinline__ void prepare_tile(const BatchTable &T, TileSmem<LPP, W> &sm, StepArgs *sa, float4 *sarr,
-                                          int busy_scene) {
-    constexpr int PT = W * 32 - PRO_FIRST;
-    const int ptid = threadIdx.x - PRO_FIRST, pl = ptid & 31, pw = ptid >> 5;
-    for (;;) {
-        if (ptid == 0) {
-            int2 e = make_int2(0, -1);
-            if (sm.pre_ok) {
-                cp_async_wait_all();
-                e = sm.pre_entry;
-            } else {  // the first call, or after an empty entry (none are listed; kept for safety)
-                const int k = atomicAdd(T.tile_next, 1);
-                if (k < sm.list_n) e = T.tile_list[k];
-            }
-            sm.pre_ok = 0;
-            sm.ntile = e.x;
-            sm.nscene = e.y;
+// The producer warp: takes the entries of the tile list (the non-empty tiles
+// of every scene) one after the other; for each it builds the tables in the
+// buffer that the compute warps have left, waits until they have read the last
+// record of the tile before, and issues the staging copies.  The next entry
+// is claimed after the copies, so its round trip is hidden.
+__device__ __forceinline__ void produce(const BatchTable &T, BlockSmem &sm, StepArgs *sa, float4 *sarr, int lane) {
+    int slot_scene[2] = {-1, -1};  // scenes whose arguments the two slots hold
+    int slot = 0;
+    int2 e = make_int2(0, -1);
+    auto claim = [&] {
+        if (lane == 0) {
+            const int k = atomicAdd(T.tile_next, 1);
+            e = k < sm.list_n ? T.tile_list[k] : make_int2(0, -1);
         }
-        pro_sync(PT);
-        const int t = sm.ntile, s = sm.nscene;
+    };
+    claim();
+#pragma unroll 1
+    for (int n = 0;; n++) {
+        const int t = __shfl_sync(0xffffffffu, e.x, 0), sd = __shfl_sync(0xffffffffu, e.y, 0);
+        const int s = sd < 0 ? -1 : sd >> 4, depth = sd & 15;
+        TileTab &tab = sm.tab[n & 1];
         if (s < 0) {
-            if (ptid == 0) sm.scene = -1;
+            if (n > 0) bar_wait<BAR_READ>();
+            if (lane == 0) tab.scene = -1;
+            bar_wait<BAR_FULL>();
             return;
         }
-        // another scene's arguments go to the second buffer (the current
-        // tile's, in the first, are in use); the main loop moves them over
-        const int buf = s == busy_scene ? 0 : 1;
-        if (buf == 1 && sm.next_args != s) {
-            const StepArgs *a0 = T.args + 2 * s;
-            const int4 *src = reinterpret_cast<const int4 *>(a0 + (a0->clk->parity & 1));
-            int4 *d = reinterpret_cast<int4 *>(sa + 1);
-            for (int k = ptid; k < int(sizeof(StepArgs) / 16); k += PT) d[k] = src[k];
-            pro_sync(PT);
-            if (ptid == 0) sm.next_args = s;
+        if (s != slot_scene[slot]) {  // the other slot: the compute warps still use this one
+            slot ^= 1;
+            if (s != slot_scene[slot]) {
+                const StepArgs *a0 = T.args + 2 * s;
+                const int4 *src = reinterpret_cast<const int4 *>(a0 + (a0->clk->parity & 1));
+                int4 *d = reinterpret_cast<int4 *>(reinterpret_cast<char *>(sa) + slot * ARGS_SIZE);
+                for (int k = lane; k < int(sizeof(StepArgs) / 16); k += 32) d[k] = src[k];
+                __syncwarp();
+                slot_scene[slot] = s;
+            }
         }
-        const StepArgs &a = sa[buf];
+        const StepArgs &a = *reinterpret_cast<const StepArgs *>(reinterpret_cast<char *>(sa) + slot * ARGS_SIZE);
         const Params &P = a.p;
         const int nx = P.gnx, ny = P.gny, nz = P.gnz;
-        const TileGeo G = tile_geo(P, t);
+        const TileGeo G = tile_geo(P, t, depth);
         const int *__restrict__ first = a.s.first;
-        {  // halo cell starts, each thread's loads in flight together
-            constexpr int NCS = (NHC * CSROW + PT - 1) / PT;
+        // halo cell starts (sorted indices), each lane's loads in flight together
+        constexpr int NCS = NHC * CSROW / 32;
+        static_assert(NHC * CSROW % 32 == 0, "whole warps of cell starts");
+        {
             int csv[NCS];
 #pragma unroll
             for (int r = 0; r < NCS; r++) {
-                const int e = ptid + r * PT;
-                const int c = e / CSROW, k = e - c * CSROW;
+                const int x = lane + r * 32;
+                const int c = x / CSROW, k = x - c * CSROW;
                 const int cx = G.X0 - 2 + c / HY, cy = G.Y0 - 2 + c % HY;
                 csv[r] = 0;
-                if (e < NHC * CSROW && k < G.nzr && cx >= 0 && cx < nx && cy >= 0 && cy < ny) {
+                if (k < G.nzr && cx >= 0 && cx < nx && cy >= 0 && cy < ny) {
                     const long long fi = (long long)(cx * ny + cy) * nz + G.zl + k;
                     if (bounds_ok(a.clk, fi, (long long)P.num_cell + 1)) csv[r] = first[fi];
                 }
             }
 #pragma unroll
-            for (int r = 0; r < NCS; r++) {
-                const int e = ptid + r * PT;
-                if (e < NHC * CSROW) (&sm.cellstart[0][0])[e] = csv[r];
-            }
+            for (int r = 0; r < NCS; r++) (&tab.cs[0][0])[lane + r * 32] = csv[r];
         }
-        pro_sync(PT);
-        if (pw == 0) {
-            // target column ranges (cells Z0 .. Z0 + depth - 1 of the 16
-            // target columns) and their prefix
-            int len = 0;
-            if (pl < NTC) {
-                const int cx = G.X0 + pl / TY, cy = G.Y0 + pl % TY;
-                int s0 = 0;
-                if (cx < nx && cy < ny && G.Z0 < nz) {
-                    const int lc = (pl / TY + 2) * HY + (pl % TY + 2);
-                    s0 = sm.cellstart[lc][G.Z0 - G.zl];
-                    len = sm.cellstart[lc][min(G.Z0 + P.tile_z - 1, nz - 1) + 1 - G.zl] - s0;
-                }
-                sm.tstart[pl] = s0;
-            }
-            const int ti = group_scan<32>(len, pl);
-            if (pl < NTC) sm.tpref[pl] = ti - len;
-            if (pl == 31) sm.tpref[NTC] = ti;
-        } else if (pw == 1) {
-            // the 64 halo columns (lane pl: columns 2 pl and 2 pl + 1), their
-            // staged offsets and the staging decision; the tile's target count
-            // (the same ranges as warp 0's) decides whether copies follow
-            int ntg = 0;
-            if (pl < NTC) {
-                const int cx = G.X0 + pl / TY, cy = G.Y0 + pl % TY;
-                if (cx < nx && cy < ny && G.Z0 < nz) {
-                    const int lc = (pl / TY + 2) * HY + (pl % TY + 2);
-                    ntg = sm.cellstart[lc][min(G.Z0 + P.tile_z - 1, nz - 1) + 1 - G.zl] -
-                          sm.cellstart[lc][G.Z0 - G.zl];
-                }
-            }
-            ntg = __reduce_add_sync(0xffffffffu, ntg);
-            int len2[2];
+        __syncwarp();
+        // the halo columns (lane l: columns 2 l and 2 l + 1), their staged offsets
+        int hs[2], hl[2];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int c = 2 * pl + h;
-                const int cx = G.X0 - 2 + c / HY, cy = G.Y0 - 2 + c % HY;
-                const bool in = cx >= 0 && cx < nx && cy >= 0 && cy < ny;
-                len2[h] = in ? sm.cellstart[c][G.nzr - 1] - sm.cellstart[c][0] : 0;
-                sm.hstart[c] = sm.cellstart[c][0];
-                // bounds-checked build: a column whose range lies outside
-                // the record arrays is counted and not staged (len 0)
-                if (!range_ok(a.clk, sm.hstart[c], len2[h], P.n_init)) len2[h] = 0;
-                sm.hlen[c] = len2[h];
-            }
-            const int v = len2[0] + len2[1];
-            const int inc = group_scan<32>(v, pl);
-            sm.hoff[2 * pl] = inc - v;
-            sm.hoff[2 * pl + 1] = inc - v + len2[0];
-            const int tot = __shfl_sync(0xffffffffu, inc, 31);
-            if (pl == 0) {
-                sm.total = tot;
-                sm.staged = tot <= CAP ? 1 : 0;
-                if (ntg > 0 && sm.staged && tot > 0)
-                    mbar_expect(&sm.bar, unsigned(tot) * unsigned(REC_N * sizeof(float4)) + unsigned(P.stage_extra));
+        for (int k = 0; k < 2; k++) {
+            const int c = 2 * lane + k;
+            hs[k] = tab.cs[c][0];
+            hl[k] = tab.cs[c][G.nzr - 1] - hs[k];
+            // bounds-checked build: a column whose range lies outside the
+            // record arrays is counted and left out
+            if (!range_ok(a.clk, hs[k], hl[k], P.n_init)) {
+                hl[k] = 0;
+                for (int q = 0; q < CSROW; q++) tab.cs[c][q] = 0;
+                hs[k] = 0;
             }
         }
-        pro_sync(PT);
-        if (sm.tpref[NTC] == 0) continue;  // an empty tile: take the next
-        if (sm.staged && sm.total > 0) {
+        // a record's staged index has the parity of its sorted index (the lanes
+        // of a target share its candidates by that parity, so its sums depend
+        // neither on the tile it falls in nor on the pruning): a column takes
+        // an even number of slots and starts at its own parity
+        const int w0 = (hl[0] + (hs[0] & 1) + 1) & ~1, w1 = (hl[1] + (hs[1] & 1) + 1) & ~1;
+        const int inc = warp_scan(w0 + w1, lane);
+        const int ho[2] = {inc - w0 - w1 + (hs[0] & 1), inc - w1 + (hs[1] & 1)};
+        const bool staged = __shfl_sync(0xffffffffu, inc, 31) <= REC_CAP;
+        const int total = __reduce_add_sync(0xffffffffu, hl[0] + hl[1]);  // records to copy
+        __syncwarp();
+        // the target columns: cells Z0 .. Z0 + depth - 1
+        int len = 0;
+        if (lane < NTC) {
+            const int cx = G.X0 + lane / TY, cy = G.Y0 + lane % TY;
+            const int *cs = tab.cs[(lane / TY + 2) * HY + (lane % TY + 2)];
+            int s0 = 0;
+            if (cx < nx && cy < ny && G.Z0 < nz) {
+                s0 = cs[G.Z0 - G.zl];
+                len = cs[min(G.Z0 + depth - 1, nz - 1) + 1 - G.zl] - s0;
+            }
+            tab.tsrt[lane] = s0;
+        }
+        const int ti = warp_scan(len, lane);
+        const int c0 = max(__ffs(__ballot_sync(0xffffffffu, len > 0)) - 1, 0);  // first column with a target
+        if (lane < NTC) tab.tpref[lane] = ti - len;
+        if (lane == 31) tab.tpref[NTC] = ti;
+        __syncwarp();
+        if (staged) {  // the cell starts as record indices
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int c = 2 * lane + k, d = ho[k] - hs[k];
+                if (hl[k] > 0)
+                    for (int q = 0; q < G.nzr; q++) tab.cs[c][q] += d;
+            }
+        }
+        __syncwarp();
+        if (lane < NTC) tab.trec[lane] = tab.cs[(lane / TY + 2) * HY + (lane % TY + 2)][max(0, min(G.Z0 - G.zl, CSROW - 1))];
+        if (lane == 0) {
+            tab.tile = t;
+            tab.depth = depth;
+            tab.scene = s;
+            tab.args = slot;
+            tab.total = total;
+            tab.staged = staged ? 1 : 0;
+            tab.nzr = G.nzr;
+            tab.rec0 = tab.cs[(c0 / TY + 2) * HY + (c0 % TY + 2)][G.Z0 - G.zl];
+            float4 org = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float md = __uint_as_float(a.clk->max_disp);
+            if (!P.full_stencil && md <= PRUNE_DISP_MAX) {
+                const float *gm = P.grid_moving ? a.clk->grid_min : P.grid_min0;
+                org = make_float4(gm[0], gm[1], gm[2], md + PRUNE_SLACK);
+            }
+            tab.org = org;
+        }
+        if (n > 0) bar_wait<BAR_READ>();
+        const bool copy = staged && total > 0;
+        if (lane == 0)
+            mbar_expect(&sm.bar, copy ? unsigned(total) * unsigned(REC_N * sizeof(float4)) + unsigned(P.stage_extra) : 0u);
+        __syncwarp();
+        if (copy) {
             // two copies a column: its P records to sarr, the interleaved rest
-            // to sarr + CAP (the record arrays are one allocation: P from
+            // to sarr + REC_CAP (the record arrays are one allocation: P from
             // f[REC_P], the rest from f[REC_P] + n_init)
             const float4 *gbase = a.r.f[REC_P];
-            for (int q = ptid; q < 2 * NHC; q += PT) {
-                const int k = q / NHC, c = q - k * NHC;
-                const int len = sm.hlen[c];
-                const int w = k == 0 ? 1 : REC_X;
-                const size_t src = (k == 0 ? 0 : size_t(P.n_init)) + size_t(sm.hstart[c]) * w;
-                const int dst = (k == 0 ? 0 : CAP) + sm.hoff[c] * w;
-                if (len > 0) bulk_to_smem(sarr + dst, gbase + src, unsigned(len * w) * unsigned(sizeof(float4)), &sm.bar);
-            }
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                if (hl[k] > 0) {
+                    bulk_to_smem(sarr + ho[k], gbase + hs[k], unsigned(hl[k]) * unsigned(sizeof(float4)), &sm.bar);
+                    bulk_to_smem(sarr + REC_CAP + ho[k] * REC_X, gbase + size_t(P.n_init) + size_t(hs[k]) * REC_X,
+                                 unsigned(hl[k] * REC_X) * unsigned(sizeof(float4)), &sm.bar);
+                }
         }
-        if (ptid == 0) {
-            sm.tile = t;
-            sm.scene = s;
-            const int k = atomicAdd(T.tile_next, 1);  // the next call's entry
-            if (k < sm.list_n) cp_async8(&sm.pre_entry, T.tile_list + k);
-            else sm.pre_entry = make_int2(0, -1);
-            sm.pre_ok = 1;
+        claim();
+        bool ok = true;
+        auto landed = [&] {
+            const long long t_wait = clock64();
+            while (!mbar_try(&sm.bar, unsigned(n & 1)))
+                if (clock64() - t_wait > WAIT_CYCLES) return false;
+            return true;
+        };
+        ok = __all_sync(0xffffffffu, landed());
+        if (!ok && lane == 0) {
+            // the copies did not complete in time: count it (the host reports
+            // MFREE_ERR_TIMEOUT); everybody leaves the kernel
+            atomicAdd(&a.clk->staging_timeouts, 1);
+            sm.fail = 1;
         }
-        return;
+        bar_wait<BAR_FULL>();
+        if (!ok) {
+            landed();  // wait once more (bounded) for the copies in flight to land
+            return;
+        }
     }
-}
-
-template <class SM> __device__ __forceinline__ void init_tile_smem(SM &sm) {
-    if (threadIdx.x == 0) {
-        mbar_init(&sm.bar, 1);
-        sm.parity = 0;
-        sm.next_args = -1;
-        sm.pre_ok = 0;
-    }
-    fence_proxy_async();
-    __syncthreads();
 }
 
 // Persistent (one block per SM) over the tiles of every scene of the table
-// (one queue).  Per tile: wait for its staged halo, then the targets in passes
-// of TCAP (rounds of all warps, then the epilogue by the threads below
-// PRO_FIRST); during the last pass's epilogue the threads from PRO_FIRST on
-// already prepare the next tile and start its staging copies.
-template <int LPP, bool CSPM, int COND, bool PREC>
-__global__ void __launch_bounds__(tile_threads<CSPM>(), 1) kb_interact(BatchTable T) {
-    constexpr int TILE_THREADS = tile_threads<CSPM>();
-    constexpr int TILE_WARPS = TILE_THREADS / 32;
-    constexpr int W = TILE_WARPS;
-    constexpr int CAP = rec_capacity<LPP, W>();
-    constexpr int G = 32 / LPP;
-    static_assert(TILE_THREADS - PRO_FIRST >= 64, "the prologue needs two warps at least");
+// (one queue).
+template <bool CSPM, int COND, bool PREC>
+__global__ void __launch_bounds__(NTHREADS, 1) kb_interact(BatchTable T) {
     extern __shared__ __align__(128) unsigned char dyn[];
-    TileSmem<LPP, W> &sm = *reinterpret_cast<TileSmem<LPP, W> *>(dyn);
-    StepArgs *sa = reinterpret_cast<StepArgs *>(dyn + args_offset<LPP, W>());
-    float4 *sarr = reinterpret_cast<float4 *>(dyn + rec_offset<LPP, W>());
+    BlockSmem &sm = *reinterpret_cast<BlockSmem *>(dyn);
+    StepArgs *sa = reinterpret_cast<StepArgs *>(dyn + ARGS_OFFSET);
+    unsigned short *queue = reinterpret_cast<unsigned short *>(dyn + QUEUE_OFFSET);
+    float4 *sarr = reinterpret_cast<float4 *>(dyn + REC_OFFSET);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / LPP, sl = lane - g * LPP;
-    if (threadIdx.x == 0) sm.list_n = *T.tile_count;
-    init_tile_smem(sm);
-    int cur = -1;
-    if (threadIdx.x >= PRO_FIRST) prepare_tile<LPP, W, CAP>(T, sm, sa, sarr, cur);
-    const StepArgs &a = sa[0];
-    for (;;) {
-        __syncthreads();  // the prepared tile's descriptor and tables are visible
-        const int s = sm.scene;
-        if (s < 0) break;
-        const int tile = sm.tile;
-        if (s != cur) {  // a new scene: its arguments wait in the second buffer
-            const int4 *src = reinterpret_cast<const int4 *>(sa + 1);
-            int4 *d = reinterpret_cast<int4 *>(sa);
-            for (int k = threadIdx.x; k < int(sizeof(StepArgs) / 16); k += blockDim.x) d[k] = src[k];
-            __syncthreads();
-            cur = s;
-        }
-        const TileGeo geo = tile_geo(a.p, tile);
-        const int X0 = geo.X0, Y0 = geo.Y0, zl = geo.zl;
-        const float4 *gbase = a.r.f[REC_P];  // tiles read from global memory: P, then the interleaved rest
-        const int gstride = a.p.n_init;
-        const int ntg = sm.tpref[NTC];
-        const bool staged = sm.staged != 0;
-        if (threadIdx.x == 0) {  // read by the targets after the next barrier
-            float4 org = make_float4(0.f, 0.f, 0.f, 0.f);
-            const float md = __uint_as_float(a.clk->max_disp);
-            if (!a.p.full_stencil && md <= PRUNE_DISP_MAX) {
-                const float *gm = a.p.grid_moving ? a.clk->grid_min : a.p.grid_min0;
-                org = make_float4(gm[0], gm[1], gm[2], md + PRUNE_SLACK);
-            }
-            sm.org = org;
-        }
-        if (staged && sm.total > 0) {
-            const unsigned par = unsigned(sm.parity);
-            const long long t_wait = clock64();
-            bool ok = true;
-            while (!mbar_try(&sm.bar, par)) {
-                if (clock64() - t_wait > WAIT_CYCLES) {
-                    ok = false;
-                    break;
-                }
-            }
-            if (!__syncthreads_and(ok)) {
-                // the copies did not complete in time: count it (the host
-                // reports MFREE_ERR_TIMEOUT), wait once more (bounded) for the
-                // copies in flight to land, and leave the kernel
-                if (threadIdx.x == 0) atomicAdd(&a.clk->staging_timeouts, 1);
-                const long long t2 = clock64();
-                while (!mbar_try(&sm.bar, par) && clock64() - t2 <= WAIT_CYCLES) {
-                }
-                cp_async_wait_all();  // the prologue's fetch of the next list entry
-                return;
-            }
-            if (threadIdx.x == 0) sm.parity ^= 1;
-        }
+    if (threadIdx.x == 0) {
+        sm.list_n = *T.tile_count;
+        sm.fail = 0;
+        mbar_init(&sm.bar, 1);
+    }
+    fence_proxy_async();
+    __syncthreads();
+    if (warp == NCOMP / 32) {
+        produce(T, sm, sa, sarr, lane);
+        return;
+    }
+    const int sl = lane % LPT;
+#pragma unroll 1
+    for (int n = 0;; n++) {
+        bar_wait<BAR_FULL>();
+        const TileTab &tab = sm.tab[n & 1];
+        if (tab.scene < 0 || sm.fail) return;
+        mbar_try(&sm.bar, unsigned(n & 1));  // the phase is complete: each thread observes the copies itself
+        const StepArgs &a = *reinterpret_cast<const StepArgs *>(reinterpret_cast<char *>(sa) + tab.args * ARGS_SIZE);
+        const int ntg = tab.tpref[NTC];
+        const bool staged = tab.staged != 0;
         // PSE: every term carries T_j - T_i, so when all staged records of the
         // tile hold the same temperature (and finite positions and volumes)
         // each term is exactly +0 and so is every target's sum; such a tile runs
         // the variant without conduction terms, on the pruned stencil, with the
-        // same results.  The test reads the staged halo after the wait.
+        // same results.
         bool pse_zero = false;
-        if (COND == MFREE_COND_PSE && staged && sm.total > 0 && !a.p.full_stencil) {
-            const float4 *rc = sarr + CAP + (REC_C - 1), *rp = sarr;
-            const float T0 = rc[0].z;
+        if (COND == MFREE_COND_PSE && staged && tab.total > 0 && !a.p.full_stencil) {
+            const float4 *rc = sarr + REC_CAP + (REC_C - 1);
+            const float T0 = rc[tab.rec0 * REC_X].z;
             bool u = true;
-            for (int k = threadIdx.x; k < sm.total; k += TILE_THREADS) {
-                const float4 c = rc[k * REC_X], p = rp[k];
-                u = u && c.z == T0 && isfinite(c.w) && isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
-            }
-            pse_zero = __syncthreads_and(u) != 0;
+            for (int hc = warp; hc < NHC; hc += NCOMP / 32)
+                for (int k = tab.cs[hc][0] + lane; k < tab.cs[hc][tab.nzr - 1]; k += 32) {
+                    const float4 c = rc[k * REC_X], p = sarr[k];
+                    u = u && c.z == T0 && isfinite(c.w) && isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+                }
+            pse_zero = compute_and(u);
             if (pse_zero && threadIdx.x == 0) atomicAdd(&a.clk->pse_zero_targets, (unsigned long long)ntg);
         }
-        for (int t0 = 0; t0 < ntg; t0 += TCAP) {
-            const int tn = min(TCAP, ntg - t0);
-            const bool last = t0 + TCAP >= ntg;
-            for (int tt = threadIdx.x; tt < tn; tt += TILE_THREADS) {
-                const int tg = t0 + tt;
-                int c = 0;
-                while (c < NTC - 1 && sm.tpref[c + 1] <= tg) c++;
-                int i = sm.tstart[c] + (tg - sm.tpref[c]);
-                if (!bounds_ok(a.clk, i, a.p.n_init)) i = 0;
-                sm.tgt[tt] = i;
-                // its cell: the z row of its column whose range holds i (the
-                // rows up to the tile's last target cell are in the table)
-                const int *cs = sm.cellstart[(c / TY + 2) * HY + (c % TY + 2)];
-                int k = geo.Z0 - zl;
-                while (cs[k + 1] <= i) k++;
-                sm.tcell[tt] = (c << 16) | (zl + k);
-            }
-            __syncthreads();
-            // rounds of TILE_WARPS * G targets; a last round with few targets
-            // left uses more lanes per target so fewer warps idle at the barrier
-            int done = 0;
 #pragma unroll 1
-            while (done < tn) {
-                const int rem = tn - done;
-                if (LPP < 32 && rem <= TILE_WARPS) {
-                    const int tt = done + warp;
-                    const bool valid = tt < tn;
-                    const int i = sm.tgt[valid ? tt : 0];
-                    if (staged && COND == MFREE_COND_PSE && pse_zero)
-                        process_target<32, CSPM, MFREE_COND_NONE, true>(a, sm, sarr, sarr, CAP, i, valid, tt, warp, 0, lane, lane, X0,
-                                                             Y0, zl);
-                    else if (staged)
-                        process_target<32, CSPM, COND, true>(a, sm, sarr, sarr, CAP, i, valid, tt, warp, 0, lane, lane, X0,
-                                                             Y0, zl);
-                    else
-                        process_target<32, CSPM, COND, false>(a, sm, sarr, gbase, gstride, i, valid, tt, warp, 0, lane, lane,
-                                                              X0, Y0, zl);
-                    done += TILE_WARPS;
-                } else if (LPP < 16 && rem <= 2 * TILE_WARPS) {
-                    const int g2 = lane >> 4, sl2 = lane & 15;
-                    const int tt = done + warp * 2 + g2;
-                    const bool valid = tt < tn;
-                    const int i = sm.tgt[valid ? tt : 0];
-                    if (staged && COND == MFREE_COND_PSE && pse_zero)
-                        process_target<16, CSPM, MFREE_COND_NONE, true>(a, sm, sarr, sarr, CAP, i, valid, tt, warp, g2, sl2, lane, X0,
-                                                             Y0, zl);
-                    else if (staged)
-                        process_target<16, CSPM, COND, true>(a, sm, sarr, sarr, CAP, i, valid, tt, warp, g2, sl2, lane, X0,
-                                                             Y0, zl);
-                    else
-                        process_target<16, CSPM, COND, false>(a, sm, sarr, gbase, gstride, i, valid, tt, warp, g2, sl2, lane,
-                                                              X0, Y0, zl);
-                    done += 2 * TILE_WARPS;
-                } else {
-                    const int tt = done + warp * G + g;
-                    const bool valid = tt < tn;
-                    const int i = sm.tgt[valid ? tt : 0];
-                    if (staged && COND == MFREE_COND_PSE && pse_zero)
-                        process_target<LPP, CSPM, MFREE_COND_NONE, true>(a, sm, sarr, sarr, CAP, i, valid, tt, warp, g, sl, lane, X0,
-                                                              Y0, zl);
-                    else if (staged)
-                        process_target<LPP, CSPM, COND, true>(a, sm, sarr, sarr, CAP, i, valid, tt, warp, g, sl, lane, X0,
-                                                              Y0, zl);
-                    else
-                        process_target<LPP, CSPM, COND, false>(a, sm, sarr, gbase, gstride, i, valid, tt, warp, g, sl, lane,
-                                                               X0, Y0, zl);
-                    done += TILE_WARPS * G;
-                }
+        for (int t0 = 0;; t0 += TCAP) {
+            float res[NRES];
+            int i = -1;
+            // targets a warp: its rounds of the pair pass (four targets each) are
+            // what a tile waits for, so few targets are spread over all warps
+            const int rounds = min(32 / LPT / 4, (min(ntg - t0, TCAP) + NCOMP / 8 - 1) / (NCOMP / 8));
+            const int tw = t0 + warp * (4 * rounds);  // the warp's first target
+            if (tw < min(ntg, t0 + TCAP)) {
+                const int tt = lane / LPT < 4 * rounds ? tw + lane / LPT : ntg;
+                if (staged && COND == MFREE_COND_PSE && pse_zero)
+                    i = process_target<CSPM, MFREE_COND_NONE, true>(a, tab, queue, sarr, ntg, tt, sl, rounds, res);
+                else if (staged)
+                    i = process_target<CSPM, COND, true>(a, tab, queue, sarr, ntg, tt, sl, rounds, res);
+                else
+                    i = process_target<CSPM, COND, false>(a, tab, queue, sarr, ntg, tt, sl, rounds, res);
             }
-            // the rounds were the last generic reads of the staged halo and the
-            // tile tables: order them before the next tile's bulk writes, which
-            // the prologue threads issue after this barrier
-            fence_proxy_async();
-            __syncthreads();
-            if (threadIdx.x < PRO_FIRST) {
-                if (threadIdx.x < tn) epilogue<PREC, COND>(a, sm.tgt[threadIdx.x], sm.res[threadIdx.x]);
-            } else if (last) {
-                prepare_tile<LPP, W, CAP>(T, sm, sa, sarr, s);
+            const bool last = t0 + TCAP >= ntg;
+            if (last) {
+                // the last reads of the staged halo: order them before the next
+                // tile's bulk writes, which the producer issues after this barrier
+                fence_proxy_async();
+                bar_arrive<BAR_READ>();
             }
-            if (!last) __syncthreads();
+            if (i >= 0 && sl == 0) epilogue<PREC, COND>(a, i, res);
+            if (last) break;
         }
     }
 }
 
 // ------------------------------------------------------------ dispatch --
-template <int LPP, bool CSPM, int COND, bool PREC> struct Variant {
+template <bool CSPM, int COND, bool PREC> struct Variant {
     static cudaError_t batch(const BatchTable &T, int grid, cudaStream_t s) {
-        auto kern = kb_interact<LPP, CSPM, COND, PREC>;
+        auto kern = kb_interact<CSPM, COND, PREC>;
         if (grid <= 0)  // prepare only: raise the shared-memory limit (outside any graph capture)
             return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-        kern<<<grid, tile_threads<CSPM>(), SMEM_LIMIT, s>>>(T);
+        kern<<<grid, NTHREADS, SMEM_LIMIT, s>>>(T);
         return cudaGetLastError();
     }
 };
 
-// calls fn(Variant<LPP, ...>{}) for the variant of the options
-template <int LPP, class F> static cudaError_t with_variant(bool cspm, int cond, bool prec, F &&fn) {
+// calls fn(Variant<...>{}) for the variant of the options
+template <class F> static cudaError_t with_variant(bool cspm, int cond, bool prec, F &&fn) {
 #define MFREE_CASE(C, CO, PR) \
-    if (cspm == C && cond == CO && prec == PR) return fn(Variant<LPP, C, CO, PR>{});
+    if (cspm == C && cond == CO && prec == PR) return fn(Variant<C, CO, PR>{});
     MFREE_CASE(false, MFREE_COND_NONE, false)
     MFREE_CASE(false, MFREE_COND_BROOKSHAW, false)
     MFREE_CASE(false, MFREE_COND_PSE, false)
@@ -1129,15 +1172,6 @@ template <int LPP, class F> static cudaError_t with_variant(bool cspm, int cond,
     MFREE_CASE(true, MFREE_COND_PSE, true)
 #undef MFREE_CASE
     return cudaErrorInvalidValue;
-}
-
-template <class F> static cudaError_t with_lpp(int lpp, bool cspm, int cond, bool prec, F &&fn) {
-    switch (lpp) {
-        case 8: return with_variant<8>(cspm, cond, prec, fn);
-        case 16: return with_variant<16>(cspm, cond, prec, fn);
-        case 32: return with_variant<32>(cspm, cond, prec, fn);
-        default: return cudaErrorInvalidValue;
-    }
 }
 
 }  // namespace mfree

@@ -81,34 +81,45 @@ struct BatchTable {
     const int *pblk;       // particle blocks of 256 threads (hash, scatter, gather, finalize)
     const int *stile;      // scan tiles of SCAN_TILE cells
     const int *cblk;       // cell blocks of 256 threads (cell fix-up)
-    const int *itile;      // pair-kernel tiles
+    const int *ibun;       // bundles of pair-kernel tiles
     int nscenes;
     int *tile_next;        // work queue of the pair kernel: next entry of tile_list (reset by kb_clock)
     int *tile_count;       // entries of tile_list (reset by kb_clock)
-    int2 *tile_list;       // non-empty pair-kernel tiles of every scene: (tile of the scene, scene)
+    int2 *tile_list;       // non-empty pair-kernel tiles of every scene: (tile of the scene, scene * 16 + depth)
 };
 
-// Pair-kernel tile = TX x TY x tile_z cells of a scene's cell grid, numbered
-// z fastest, then y, then x
+// Pair-kernel tiles.  A bundle is TX x TY columns of a scene's cell grid
+// (numbered y fastest); the tile list cuts its levels along z into tiles of up
+// to Params::tile_z levels and tile_cap targets, skipping empty levels.  So
+// tiles come out about equally full, at the surfaces of a block and in dense
+// or thin regions too (tiles of a fixed depth held 156 targets of the 211 of a
+// full one on the 1M-particle block).
+// A tile is named by bundle * gnz + its first level, and its depth.
 constexpr int TX = 4, TY = 4;
+constexpr int TILE_HALO_MAX = 1640;  // records the halo of a tile should hold at most (estimated from its bundle)
 struct TileGeo {
-    int X0, Y0, Z0, zl, nzr;
+    int X0, Y0, Z0, zl, nzr, depth;
 };
-__host__ __device__ __forceinline__ TileGeo tile_geo(const Params &P, int t) {
-    const int TZ = P.tile_z;
-    const int nty = (P.gny + TY - 1) / TY, ntz = (P.gnz + TZ - 1) / TZ;
-    const int tz = t % ntz, txy = t / ntz, ty = txy % nty, tx = txy / nty;
+__host__ __device__ __forceinline__ TileGeo tile_geo(const Params &P, int t, int depth) {
+    const int nby = (P.gny + TY - 1) / TY;
+    const int b = t / P.gnz;
     TileGeo g;
-    g.X0 = tx * TX;
-    g.Y0 = ty * TY;
-    g.Z0 = tz * TZ;
+    g.X0 = b / nby * TX;
+    g.Y0 = b % nby * TY;
+    g.Z0 = t - b * P.gnz;
+    g.depth = depth;
     g.zl = g.Z0 - 2 > 0 ? g.Z0 - 2 : 0;
-    const int zh = g.Z0 + TZ + 1 < P.gnz - 1 ? g.Z0 + TZ + 1 : P.gnz - 1;
+    const int zh = g.Z0 + depth + 1 < P.gnz - 1 ? g.Z0 + depth + 1 : P.gnz - 1;
     g.nzr = zh - g.zl + 2;  // cell starts per halo column of the tile (inclusive end)
     return g;
 }
-__host__ __device__ __forceinline__ int num_tiles(const Params &P) {
-    return ((P.gnx + TX - 1) / TX) * ((P.gny + TY - 1) / TY) * ((P.gnz + P.tile_z - 1) / P.tile_z);
+__host__ __device__ __forceinline__ int num_bundles(const Params &P) {
+    return ((P.gnx + TX - 1) / TX) * ((P.gny + TY - 1) / TY);
+}
+// an upper bound of a scene's tiles: a tile ends at the depth limit, at the
+// end of its bundle, or because it and its successor hold more than tile_cap
+inline long long max_tiles(const Params &P) {
+    return (long long)num_bundles(P) * (P.gnz / P.tile_z + 2) + 2ll * P.n_init / P.tile_cap + 2;
 }
 
 // scene of block x: the last s with prefix[s] <= x (prefix has nscenes + 1 entries)
@@ -150,8 +161,8 @@ __global__ void kb_finalize(BatchTable T);
 __global__ void kb_force_final(BatchTable T);
 // one pair-kernel launch over the tiles of every scene (all scenes share the
 // variant); grid <= 0 only prepares the variant
-cudaError_t launch_interact_batch(const BatchTable &T, int lanes_per_particle, bool cspm, int conduction,
-                                  bool precision, int grid, cudaStream_t s);
+cudaError_t launch_interact_batch(const BatchTable &T, bool cspm, int conduction, bool precision, int grid,
+                                  cudaStream_t s);
 
 // the sort kernels on arguments passed by value, for the allocation-free
 // cell-list build (mfree_static.cu)

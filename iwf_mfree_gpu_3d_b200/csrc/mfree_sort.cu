@@ -325,39 +325,69 @@ __device__ __forceinline__ void cell_fixup_body(const StepArgs &a, int bid) {
 }
 __global__ void __launch_bounds__(256) k_cell_fixup(StepArgs a) { cell_fixup_body(a, blockIdx.x); }
 
-// The pair kernel's list of non-empty tiles: one thread per tile of every
-// scene; a tile with a particle in one of its target cells is appended as
-// (tile of its scene, scene), one atomic per warp.  The order of the list
-// changes which block runs a tile, never a result.
-__device__ __forceinline__ void tile_list_body(const BatchTable &T, int g) {
-    const int total = T.itile[T.nscenes];
-    bool ne = false;
-    int s = 0, t = 0;
-    if (g < total) {
-        s = find_scene(T.itile, T.nscenes, g);
-        t = g - T.itile[s];
-        const StepArgs *a0 = T.args + 2 * s;
-        const StepArgs &a = a0[a0->clk->parity & 1];
-        const Params &P = a.p;
-        const int nx = P.gnx, ny = P.gny, nz = P.gnz;
-        const TileGeo G = tile_geo(P, t);
-        const int zend = min(G.Z0 + P.tile_z - 1, nz - 1) + 1;
-        const int *__restrict__ first = a.s.first;
+// The pair kernel's list of non-empty tiles: one warp per bundle of every
+// scene.  Lane k holds the targets below level base + k of the bundle, so a
+// tile's depth is one ballot over the lanes behind its first level; the
+// bundle's tiles are appended with one atomic per 32 of them.  The order of
+// the list changes which block runs a tile, never a result.
+__device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int lane) {
+    if (g >= T.ibun[T.nscenes]) return;
+    const int s = find_scene(T.ibun, T.nscenes, g);
+    const int bun = g - T.ibun[s];
+    const StepArgs &a = scene_args(T, s);
+    const Params &P = a.p;
+    const int nx = P.gnx, ny = P.gny, nz = P.gnz;
+    const TileGeo G = tile_geo(P, bun * nz, 1);
+    const int *__restrict__ first = a.s.first;
+    int base = 0, F = 0;
+    auto load = [&](int z) {  // F = targets of the bundle below level z + lane, up to a constant
+        base = z;
+        F = 0;
+        const int zz = min(z + lane, nz);
+#pragma unroll
         for (int c = 0; c < TX * TY; c++) {
             const int cx = G.X0 + c / TY, cy = G.Y0 + c % TY;
-            if (cx < nx && cy < ny && G.Z0 < nz) {
-                const int cb = (cx * ny + cy) * nz;
-                ne |= first[cb + zend] > first[cb + G.Z0];
-            }
+            if (cx < nx && cy < ny) F += first[(cx * ny + cy) * nz + zz];
         }
+    };
+    auto at = [&](int z) { return __shfl_sync(0xffffffffu, F, min(z, nz) - base); };
+    load(0);
+    int2 mine = make_int2(0, 0);
+    int n = 0;
+    auto flush = [&] {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(T.tile_count, n);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (lane < n) T.tile_list[k + lane] = mine;
+        n = 0;
+    };
+    for (int z0 = 0; z0 < nz;) {
+        if (min(z0 + TILE_Z_MAX + 2, nz) > base + 31) load(max(z0 - 2, 0));
+        // the first level with a target (a level past the window: look again there)
+        const int below = at(z0);
+        const unsigned some = __ballot_sync(0xffffffffu, base + lane > z0 && base + lane <= nz && F > below);
+        if (some == 0) {
+            z0 = base + 31;
+            continue;
+        }
+        const int zf = base + __ffs(some) - 2;
+        if (zf > z0) {
+            z0 = zf;
+            continue;  // (the window may have to move)
+        }
+        // lane d: would a tile of depth d fit?  Its halo is estimated as four
+        // times the bundle's own particles in the halo's levels.
+        const int d = lane;
+        const int in = __shfl_sync(0xffffffffu, F, min(max(min(z0 + d, nz) - base, 0), 31)) - below;
+        const int lo = at(max(z0 - 2, 0)), hi = __shfl_sync(0xffffffffu, F, min(max(min(z0 + d + 2, nz) - base, 0), 31));
+        const bool no = d > P.tile_z || z0 + d > nz || in > P.tile_cap || 4 * (hi - lo) > TILE_HALO_MAX;
+        const unsigned bad = __ballot_sync(0xffffffffu, no && d > 1);
+        const int depth = bad ? __ffs(bad) - 2 : 1;
+        if (lane == n) mine = make_int2(bun * nz + z0, s * 16 + depth);
+        if (++n == 32) flush();
+        z0 += depth;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, ne);
-    if (m == 0) return;
-    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(T.tile_count, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (ne) T.tile_list[base + __popc(m & ((1u << lane) - 1u))] = make_int2(t, s);
+    if (n > 0) flush();
 }
 
 // blocks past the cell blocks of every scene build the tile list (the cell
@@ -365,7 +395,7 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g) {
 __global__ void __launch_bounds__(256) kb_cell_fixup(BatchTable T) {
     const int nb = T.cblk[T.nscenes];
     if (int(blockIdx.x) >= nb) {
-        tile_list_body(T, (int(blockIdx.x) - nb) * 256 + int(threadIdx.x));
+        tile_list_body(T, (int(blockIdx.x) - nb) * 8 + int(threadIdx.x >> 5), int(threadIdx.x & 31));
         return;
     }
     run_batched(T, T.cblk, [](const StepArgs &a, int b) { cell_fixup_body(a, b); });
@@ -425,10 +455,10 @@ template <bool PREC> __device__ __forceinline__ void gather_predict_body(const S
     r.f[REC_P][i] = make_float4(hs.x, hs.y, hs.z, fc.w);  // raw tool_particle value
     float4 *x = r.f[REC_V] + size_t(i) * REC_X;  // V, A, B, R, C interleaved
     x[REC_V - 1] = make_float4(hs.vx, hs.vy, hs.vz, hs.rho);
-    x[REC_A - 1] = make_float4((hs.S[0] - prs) * ir2, (hs.S[1] - prs) * ir2, (hs.S[2] - prs) * ir2, hs.S[3] * ir2);
-    x[REC_B - 1] = make_float4(hs.S[4] * ir2, hs.S[5] * ir2, sqrtf(P.K / hs.rho), pos.w);
-    x[REC_R - 1] = make_float4(Rr[0], Rr[1], Rr[2], Rr[3]);
-    x[REC_C - 1] = make_float4(Rr[4], Rr[5], hs.T, P.mass / hs.rho);
+    x[REC_A - 1] = make_float4((hs.S[0] - prs) * ir2, hs.S[3] * ir2, hs.S[4] * ir2, hs.S[5] * ir2);
+    x[REC_B - 1] = make_float4((hs.S[1] - prs) * ir2, (hs.S[2] - prs) * ir2, sqrtf(P.K / hs.rho), pos.w);
+    x[REC_R - 1] = make_float4(Rr[0], Rr[3], Rr[4], Rr[5]);
+    x[REC_C - 1] = make_float4(Rr[1], Rr[2], hs.T, P.mass / hs.rho);
     if (P.diagnostics) a.s.pos_half[i] = make_float4(hs.x, hs.y, hs.z, 0.f);
 }
 template <bool PREC> __global__ void __launch_bounds__(256) kb_gather_predict(BatchTable T) {

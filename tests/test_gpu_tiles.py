@@ -1,0 +1,80 @@
+"""The pair kernel's tiles: where the grid is cut must not show in the results.
+
+A target's candidates are shared between its two lanes by the parity of their
+sorted index, and its sums are joined in a fixed order, so they are the same
+bits for every tile depth, for tiles that hold more targets than a block
+serves at once, for halos read from global memory instead of shared memory and
+for neighbour queues that overflow -- and the same in a batch, whose tiles are
+sized by the particles of all its scenes.
+"""
+import numpy as np
+import pytest
+
+from iwf_mfree_gpu_3d_b200 import api, scenes
+
+from helpers import loaded
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("POS", "VEL", "S", "T", "EPS_PL", "RHO", "POS_T", "VEL_T", "S_T", "T_T", "FC", "NUM_NBH", "ID")
+
+
+def _state(sc, steps, **opt):
+    sim = api.Simulation.from_scene(sc, diagnostics=1, **opt)
+    if hasattr(sc, "S0"):
+        sim.set("S", sc.S0)
+    sim.advance(steps, record_every=1)
+    out = {n: sim.get(n) for n in NAMES}
+    out["forces"] = sim.tool_forces()
+    c = sim.counters()
+    assert c["staging_timeouts"] == 0 and c["bounds_errors"] == 0
+    sim.close()
+    return out
+
+
+def _same(a, b, what):
+    for n in a:
+        np.testing.assert_array_equal(a[n], b[n], err_msg=f"{what}: {n}")
+
+
+def _dense(sc, f):
+    """The scene's particles drawn together by f in y: more neighbours than a
+    queue holds and, at the smaller f, halos beyond the staging area."""
+    sc.pos[:, 1] *= np.float32(f)
+    return sc
+
+
+CASES = {
+    # one cell column and ragged edges: tiles of a few targets
+    "ragged": lambda: scenes.orthogonal_cutting(29, 7, 5, conduction=0),
+    "cspm_pse": lambda: loaded(scenes.orthogonal_cutting(23, 17, 13, cspm=True, conduction=2)),
+    "cspm_brookshaw": lambda: loaded(scenes.orthogonal_cutting(23, 17, 13, cspm=True, conduction=1, precision=1)),
+    "overflow": lambda: _dense(scenes.orthogonal_cutting(26, 20, 12, conduction=1), 0.6),
+    "from_global": lambda: _dense(scenes.orthogonal_cutting(26, 40, 12, cspm=True, conduction=2), 0.2),
+}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_results_do_not_depend_on_the_tiles(case):
+    ref = _state(CASES[case](), 3)
+    if case in ("overflow", "from_global"):
+        assert ref["NUM_NBH"].max() > 96  # beyond a queue's capacity
+    for depth in (1, 2, 5, 7):
+        _same(ref, _state(CASES[case](), 3, tile_depth=depth), f"{case}, depth {depth}")
+
+
+def test_results_do_not_depend_on_the_batch_around_a_scene():
+    # alone its tiles hold 32 targets at most; beside the larger scene they are fuller
+    small = lambda: scenes.orthogonal_cutting(18, 9, 7, precision=1)  # noqa: E731
+    big = scenes.orthogonal_cutting(80, 40, 20, precision=1)
+    b = api.Batch()
+    sims = [api.Simulation.from_scene(sc) for sc in (small(), big)]
+    for s in sims:
+        b.admit(s)
+    b.step(4, record_every=1)
+    ref = api.Simulation.from_scene(small())
+    ref.advance(4, record_every=1)
+    for n in ("POS", "VEL", "S", "T", "VEL_T", "ID"):
+        np.testing.assert_array_equal(sims[0].get(n), ref.get(n), err_msg=n)
+    ref.close()
+    b.close()
