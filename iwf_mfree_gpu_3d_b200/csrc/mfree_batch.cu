@@ -179,8 +179,8 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     cudaError_t e = launch_gather_predict_batch(T, b->prec, b->tot_pblk, s);
     if (e == cudaSuccess) e = launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s);
     if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));
-    kb_finalize<<<b->tot_pblk, 256, 0, s>>>(T);
-    kb_force_final<<<n, 256, 0, s>>>(T);
+    kb_finalize<<<b->tot_pblk, FIN_BLOCK, 0, s>>>(T);
+    if (record_mode == 1 || (record_mode == 2 && b->table_record_every > 0)) kb_force_final<<<n, 256, 0, s>>>(T);
     CUDA_TRY(cudaGetLastError());
     return MFREE_OK;
 }

@@ -175,6 +175,7 @@ struct Scratch {
     int *nnb;              // neighbour counts (diagnostics)
     float4 *pos_half;      // half-step positions (diagnostics)
     float4 *nrm;           // contact normal (diagnostics)
+    unsigned *contact;     // bitmap of the particles inside a tool box: set by the pair kernel, cleared by kb_finalize
     float *force_part;     // per-block partial tool forces (3 per tool per block)
     float *forces;         // per-tool force of the last recorded step (3 per tool)
 };

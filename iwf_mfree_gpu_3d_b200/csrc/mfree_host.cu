@@ -386,8 +386,10 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     if (le == cudaSuccess)
         run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
     if (le != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(le));
-    run(9, [&] { kb_finalize<<<nb, 256, 0, s>>>(T); });
-    if (!c->tools.empty()) run(10, [&] { kb_force_final<<<1, 256, 0, s>>>(T); });
+    run(9, [&] { kb_finalize<<<finalize_blocks(c->n_init), FIN_BLOCK, 0, s>>>(T); });
+    // (a step that cannot record needs no sum of the recorded forces)
+    if (!c->tools.empty() && (record_mode == 1 || (record_mode == 2 && record_every > 0)))
+        run(10, [&] { kb_force_final<<<1, 256, 0, s>>>(T); });
     CUDA_TRY(cudaGetLastError());
     return MFREE_OK;
 }
@@ -479,6 +481,7 @@ int alloc_ctx(int n, cudaStream_t stream, std::unique_ptr<mfree_ctx> &out) {
     if ((st = dalloc(c.get(), &c->scr.nnb, n, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.pos_half, n, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.nrm, n, L))) return bail(st);
+    if ((st = dalloc(c.get(), &c->scr.contact, size_t(n + 31) / 32, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.force_part, size_t((n + 255) / 256) * 3 * MAX_TOOLS, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->d_clk, 1, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->d_forces, 3 * MAX_TOOLS, L))) return bail(st);
@@ -486,6 +489,7 @@ int alloc_ctx(int n, cudaStream_t stream, std::unique_ptr<mfree_ctx> &out) {
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_clk, 0, sizeof(DevClock), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_forces, 0, sizeof(float) * 3 * MAX_TOOLS, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.contact, 0, sizeof(unsigned) * (size_t(n + 31) / 32), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.nnb, 0, sizeof(int) * n, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.pos_half, 0, sizeof(float4) * n, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.nrm, 0, sizeof(float4) * n, c->stream);
@@ -501,7 +505,7 @@ size_t scene_bytes(int n, long long num_cell) {
     const long long tiles = (num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE;
     size_t t = 26 * b(n, sizeof(float4)) + b(REC_N * (long long)n, sizeof(float4));
     t += 3 * b(n, sizeof(int)) + b(hb + 1, sizeof(int)) + b(n, sizeof(int)) + 2 * b(n, sizeof(float4));
-    t += b(fb * 3 * MAX_TOOLS, sizeof(float)) + b(1, sizeof(DevClock)) + b(3 * MAX_TOOLS, sizeof(float));
+    t += b((n + 31) / 32, sizeof(unsigned)) + b(fb * 3 * MAX_TOOLS, sizeof(float)) + b(1, sizeof(DevClock)) + b(3 * MAX_TOOLS, sizeof(float));
     t += b(num_cell + 1, sizeof(int)) + b(num_cell + 2 + SCAN_TILE, sizeof(int)) + b(tiles + 1, sizeof(int));
     t += b(num_cell + 1, sizeof(int2));
     t += single_table_bytes();

@@ -513,6 +513,7 @@ __device__ void epilogue(const StepArgs &a, int i, const float *res) {
     }
     // ---- contact reset; particles inside a tool box finish in kb_finalize
     const bool deferred = !tool && contact_candidate(a, pos.x, pos.y, pos.z);
+    if (deferred) atomicOr(&a.s.contact[i >> 5], 1u << (i & 31));
     fc.x = fc.y = fc.z = 0.f;  // w keeps tool_p
     ft.x = ft.y = ft.z = 0.f;  // w keeps blanked
     if (!deferred) {
