@@ -50,14 +50,14 @@ struct mfree_batch {
     bool variant_set = false, cspm = false, prec = false;
     int cond = 0;
     std::vector<Slot> slots;
-    // device table: StepArgs[2 cap] | 4 prefixes of cap + 1 ints | queue counter
+    // device table: StepArgs[2 cap] | 3 prefixes of cap + 1 ints | queue counters
     void *d_table = nullptr;
     int cap = 0;
     int2 *d_tiles = nullptr;  // the pair kernel's tile list over every scene
     long long tiles_cap = 0;
     BatchTable T{};
     std::vector<int> run;  // slots in the table, in table order
-    int tot_pblk = 0, tot_stile = 0, tot_cblk = 0, tot_ibun = 0;
+    int tot_pblk = 0, tot_stile = 0, tot_ibun = 0;
     bool dirty = true;
     int table_record_every = -1;
     cudaGraphExec_t graph = nullptr;
@@ -67,7 +67,7 @@ struct mfree_batch {
 namespace {
 
 size_t table_bytes(int cap) {
-    return sizeof(StepArgs) * 2 * size_t(cap) + sizeof(int) * (4 * size_t(cap + 1) + 2);
+    return sizeof(StepArgs) * 2 * size_t(cap) + sizeof(int) * (3 * size_t(cap + 1) + 2);
 }
 
 void drop_graph(mfree_batch *b) {
@@ -102,13 +102,12 @@ int build_table(mfree_batch *b, int record_every) {
     b->T.args = dargs;
     b->T.pblk = dint;
     b->T.stile = dint + (b->cap + 1);
-    b->T.cblk = dint + 2 * (b->cap + 1);
-    b->T.ibun = dint + 3 * (b->cap + 1);
-    b->T.tile_next = dint + 4 * (b->cap + 1);
-    b->T.tile_count = dint + 4 * (b->cap + 1) + 1;
+    b->T.ibun = dint + 2 * (b->cap + 1);
+    b->T.tile_next = dint + 3 * (b->cap + 1);
+    b->T.tile_count = dint + 3 * (b->cap + 1) + 1;
     std::vector<StepArgs> args(2 * size_t(n));
-    std::vector<int> pre(4 * size_t(b->cap + 1), 0);
-    int *pb = pre.data(), *ps = pb + (b->cap + 1), *pc = ps + (b->cap + 1), *pt = pc + (b->cap + 1);
+    std::vector<int> pre(3 * size_t(b->cap + 1), 0);
+    int *pb = pre.data(), *ps = pb + (b->cap + 1), *pt = ps + (b->cap + 1);
     long long particles = 0, tiles = 0;
     for (int k : b->run) particles += b->slots[k].c->n_init;
     const int cap_targets = default_tile_cap(particles, b->num_sms);
@@ -135,13 +134,11 @@ int build_table(mfree_batch *b, int record_every) {
         const Params &P = args[2 * s].p;
         pb[s + 1] = pb[s] + hash_blocks(c);
         ps[s + 1] = ps[s] + scan_tiles(c);
-        pc[s + 1] = pc[s] + int((c->num_cell + 255) / 256);
         pt[s + 1] = pt[s] + num_bundles(P);
         tiles += max_tiles(P);
     }
     b->tot_pblk = pb[n];
     b->tot_stile = ps[n];
-    b->tot_cblk = pc[n];
     b->tot_ibun = pt[n];
     if (tiles > b->tiles_cap) {  // the tile list of all scenes
         CUDA_TRY(cudaStreamSynchronize(b->stream));  // the old list may still be read
@@ -171,11 +168,8 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     const int n = T.nscenes;
     kb_clock<<<(n + 127) / 128, 128, 0, s>>>(T, record_mode);
     kb_hash<<<b->tot_pblk, HASH_BLOCK, 0, s>>>(T);
-    kb_scan_reduce<<<b->tot_stile, SCAN_THREADS, 0, s>>>(T);
-    kb_scan_top<<<n, 1024, 0, s>>>(T);
-    kb_scan_down<<<b->tot_stile, SCAN_THREADS, 0, s>>>(T);
-    kb_scatter<<<b->tot_pblk, HASH_BLOCK, 0, s>>>(T);
-    kb_cell_fixup<<<b->tot_cblk + (b->tot_ibun + 7) / 8, 256, 0, s>>>(T);
+    kb_scan<<<b->tot_stile, SCAN_THREADS, 0, s>>>(T);
+    kb_scatter<<<b->tot_pblk + (b->tot_ibun + 7) / 8, HASH_BLOCK, 0, s>>>(T);
     cudaError_t e = launch_gather_predict_batch(T, b->prec, b->tot_pblk, s);
     if (e == cudaSuccess) e = launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s);
     if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));

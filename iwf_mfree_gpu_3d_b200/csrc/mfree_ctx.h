@@ -42,8 +42,7 @@ struct TraceRange {
 };
 // the step's kernels in launch order (the ids of mfree_get_kernel_times)
 constexpr const char *KERNEL_TRACE_NAMES[MFREE_NUM_KERNELS] = {
-    "kb_clock", "kb_hash", "kb_scan_reduce", "kb_scan_top", "kb_scan_down", "kb_scatter",
-    "kb_cell_fixup", "kb_gather_predict", "kb_interact", "kb_finalize", "kb_force_final"};
+    "kb_clock", "kb_hash", "", "", "kb_scan", "kb_scatter", "", "kb_gather_predict", "kb_interact", "kb_finalize", "kb_force_final"};
 
 struct DevTool {
     HostTool host;
@@ -153,7 +152,7 @@ int clone_ctx(const mfree_ctx *c, cudaStream_t s, std::unique_ptr<mfree_ctx> &ou
 // waits for and frees the context's output job (mfree_output.cu)
 int finish_output(mfree_ctx *c, bool release);
 size_t scene_bytes(int n, long long num_cell);
-inline size_t single_table_bytes() { return 2 * sizeof(mfree::StepArgs) + 10 * sizeof(int); }
+inline size_t single_table_bytes() { return 2 * sizeof(mfree::StepArgs) + 8 * sizeof(int); }
 // device memory the context holds, in bytes
 size_t device_bytes(const mfree_ctx *c);
 

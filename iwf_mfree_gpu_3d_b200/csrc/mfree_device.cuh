@@ -168,10 +168,12 @@ struct Scratch {
     unsigned *key;         // cell id per particle (num_cell = blanked), current order
     unsigned *key_sorted;  // cell id in sorted order
     int *perm;             // sorted position -> previous position
+    int *perm_raw;         // the same before a cell's entries are in order
     int *count;            // num_cell + 1 counters
     int *first;            // exclusive scan of count: num_cell + 2 entries
-    int *tile_sum;         // per-tile sums of the scan
-    int *blank_block;      // blanked particles per hash block, scanned in place
+    int *tile_sum;         // particles per tile of the scan (added by the hash, zeroed by the scatter)
+    int *blank_block;      // blanked particles per hash block
+    int *blank_group;      // and per BLANK_GROUP of them (zeroed by the gather)
     int *nnb;              // neighbour counts (diagnostics)
     float4 *pos_half;      // half-step positions (diagnostics)
     float4 *nrm;           // contact normal (diagnostics)

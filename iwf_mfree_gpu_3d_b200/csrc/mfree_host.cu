@@ -7,7 +7,7 @@
 // blanking.cpp), leap_frog::step (leap_frog.cu:121-195) and the process globals
 // of mfree_gpu_3d.cpp:41-48.
 //
-// A step is 11 kernels on one stream with no host synchronisation (N lives on
+// A step is 8 kernels at most on one stream with no host synchronisation (N lives on
 // the device), so it can also be captured once into a CUDA graph and replayed.
 #include <climits>
 #include <cstdint>
@@ -178,6 +178,7 @@ Params make_params(const mfree_ctx *c) {
     return P;
 }
 
+static int blank_groups(int n) { return (n + HASH_BLOCK * BLANK_GROUP - 1) / (HASH_BLOCK * BLANK_GROUP); }
 int hash_blocks(const mfree_ctx *c) { return (c->n_init + HASH_BLOCK - 1) / HASH_BLOCK; }
 int scan_tiles(const mfree_ctx *c) { return int((c->num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE); }
 
@@ -234,6 +235,7 @@ int ensure_scratch(mfree_ctx *c) {
     // the pair kernel's tile list: a tile of any depth holds a cell at least
     if ((st = dalloc(c, &c->d_tiles, cells + 1, L))) return st;
     CUDA_TRY(cudaMemsetAsync(c->scr.count, 0, sizeof(int) * (cells + 1), c->stream));
+    CUDA_TRY(cudaMemsetAsync(c->scr.tile_sum, 0, sizeof(int) * ((cells + 1 + SCAN_TILE - 1) / SCAN_TILE + 1), c->stream));
     c->scratch_cells = size_t(cells);
     invalidate_graphs(c);
     return MFREE_OK;
@@ -329,7 +331,7 @@ int ensure_table(mfree_ctx *c, int record_every) {
     c->cur = keep;
     const Params &P = args[0].p;
     const int nbun = num_bundles(P);
-    const int pre[10] = {0, hash_blocks(c), 0, scan_tiles(c), 0, int((c->num_cell + 255) / 256), 0, nbun, 0, 0};
+    const int pre[8] = {0, hash_blocks(c), 0, scan_tiles(c), 0, nbun, 0, 0};
     StepArgs *da = (StepArgs *)c->d_table;
     int *di = (int *)(da + 2);
     // pageable sources: the call returns once the bytes are staged
@@ -338,10 +340,9 @@ int ensure_table(mfree_ctx *c, int record_every) {
     c->T.args = da;
     c->T.pblk = di;
     c->T.stile = di + 2;
-    c->T.cblk = di + 4;
-    c->T.ibun = di + 6;
-    c->T.tile_next = di + 8;
-    c->T.tile_count = di + 9;
+    c->T.ibun = di + 4;
+    c->T.tile_next = di + 6;
+    c->T.tile_count = di + 7;
     c->T.tile_list = c->d_tiles;
     c->T.nscenes = 1;
     c->nbun = nbun;
@@ -377,11 +378,8 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     };
     run(0, [&] { kb_clock<<<1, 32, 0, s>>>(T, record_mode); });
     run(1, [&] { kb_hash<<<hb, HASH_BLOCK, 0, s>>>(T); });
-    run(2, [&] { kb_scan_reduce<<<tiles, SCAN_THREADS, 0, s>>>(T); });
-    run(3, [&] { kb_scan_top<<<1, 1024, 0, s>>>(T); });
-    run(4, [&] { kb_scan_down<<<tiles, SCAN_THREADS, 0, s>>>(T); });
-    run(5, [&] { kb_scatter<<<hb, HASH_BLOCK, 0, s>>>(T); });
-    run(6, [&] { kb_cell_fixup<<<int((c->num_cell + 255) / 256) + (c->nbun + 7) / 8, 256, 0, s>>>(T); });
+    run(4, [&] { kb_scan<<<tiles, SCAN_THREADS, 0, s>>>(T); });
+    run(5, [&] { kb_scatter<<<hb + (c->nbun + 7) / 8, HASH_BLOCK, 0, s>>>(T); });
     run(7, [&] { le = launch_gather_predict_batch(T, P.precision != 0, nb, s); });
     if (le == cudaSuccess)
         run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
@@ -477,6 +475,8 @@ int alloc_ctx(int n, cudaStream_t stream, std::unique_ptr<mfree_ctx> &out) {
     if ((st = dalloc(c.get(), &c->scr.key, n, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.key_sorted, n, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.perm, n, L))) return bail(st);
+    if ((st = dalloc(c.get(), &c->scr.perm_raw, n, L))) return bail(st);
+    if ((st = dalloc(c.get(), &c->scr.blank_group, blank_groups(n), L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.blank_block, (n + HASH_BLOCK - 1) / HASH_BLOCK + 1, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.nnb, n, L))) return bail(st);
     if ((st = dalloc(c.get(), &c->scr.pos_half, n, L))) return bail(st);
@@ -490,6 +490,7 @@ int alloc_ctx(int n, cudaStream_t stream, std::unique_ptr<mfree_ctx> &out) {
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_clk, 0, sizeof(DevClock), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_forces, 0, sizeof(float) * 3 * MAX_TOOLS, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.contact, 0, sizeof(unsigned) * (size_t(n + 31) / 32), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.blank_group, 0, sizeof(int) * blank_groups(n), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.nnb, 0, sizeof(int) * n, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.pos_half, 0, sizeof(float4) * n, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->scr.nrm, 0, sizeof(float4) * n, c->stream);
@@ -504,7 +505,7 @@ size_t scene_bytes(int n, long long num_cell) {
     const long long hb = (n + HASH_BLOCK - 1) / HASH_BLOCK, fb = (n + 255) / 256;
     const long long tiles = (num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE;
     size_t t = 26 * b(n, sizeof(float4)) + b(REC_N * (long long)n, sizeof(float4));
-    t += 3 * b(n, sizeof(int)) + b(hb + 1, sizeof(int)) + b(n, sizeof(int)) + 2 * b(n, sizeof(float4));
+    t += 4 * b(n, sizeof(int)) + b(blank_groups(n), sizeof(int)) + b(hb + 1, sizeof(int)) + b(n, sizeof(int)) + 2 * b(n, sizeof(float4));
     t += b((n + 31) / 32, sizeof(unsigned)) + b(fb * 3 * MAX_TOOLS, sizeof(float)) + b(1, sizeof(DevClock)) + b(3 * MAX_TOOLS, sizeof(float));
     t += b(num_cell + 1, sizeof(int)) + b(num_cell + 2 + SCAN_TILE, sizeof(int)) + b(tiles + 1, sizeof(int));
     t += b(num_cell + 1, sizeof(int2));

@@ -9,6 +9,7 @@
 namespace mfree {
 
 constexpr int HASH_BLOCK = 256;
+constexpr int BLANK_GROUP = 128;  // hash blocks per group of blanked counts
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
@@ -87,7 +88,6 @@ struct BatchTable {
     const StepArgs *args;  // [2 s + parity]
     const int *pblk;       // particle blocks of 256 threads (hash, scatter, gather, finalize)
     const int *stile;      // scan tiles of SCAN_TILE cells
-    const int *cblk;       // cell blocks of 256 threads (cell fix-up)
     const int *ibun;       // bundles of pair-kernel tiles
     int nscenes;
     int *tile_next;        // work queue of the pair kernel: next entry of tile_list (reset by kb_clock)
@@ -156,13 +156,50 @@ __device__ __forceinline__ void load_scene_args(StepArgs &dst, const BatchTable 
     for (int k = threadIdx.x; k < int(sizeof(StepArgs) / 16); k += blockDim.x) d[k] = src[k];
 }
 
+// Adds a block's particles to the counts of their cells (counted: a thread's
+// cell, all ones for none) and to the sums of the scan's tiles.  Particles come
+// in last step's sorted order, so a warp's cells run in stretches: the first
+// lane of each adds its length (about 14 atomics a warp instead of 32).  A
+// block's particles lie in one or two tiles: it adds them up in shared memory
+// for the tiles around its middle thread's, and once to memory (an atomic a
+// warp on the few tile sums took 13 us on 1M particles).
+__device__ __forceinline__ void count_cells(const StepArgs &a, unsigned counted) {
+    constexpr unsigned NEAR = 32;
+    __shared__ int near_sum[NEAR];
+    __shared__ unsigned near0;
+    const int lane = threadIdx.x & 31;
+    const unsigned none = 0xffffffffu, tile = counted == none ? none : counted / SCAN_TILE;
+    if (threadIdx.x < NEAR) near_sum[threadIdx.x] = 0;
+    if (threadIdx.x == HASH_BLOCK / 2) near0 = tile == none ? none : max(tile, NEAR / 2) - NEAR / 2;
+    __syncthreads();
+    const unsigned n0 = near0;
+    auto stretches = [&](unsigned v, auto &&add) {
+        const unsigned prev = __shfl_up_sync(0xffffffffu, v, 1);
+        const bool start = lane == 0 || prev != v;
+        const unsigned starts = __ballot_sync(0xffffffffu, start);
+        if (start && v != none) {
+            const unsigned after = starts & ~((2u << lane) - 1u);
+            add(v, (after ? __ffs(after) - 1 : 32) - lane);
+        }
+    };
+    stretches(counted, [&](unsigned v, int n) { atomicAdd(a.s.count + v, n); });
+    stretches(tile, [&](unsigned v, int n) {
+        if (n0 != none && v - n0 < NEAR) atomicAdd(&near_sum[v - n0], n);
+        else atomicAdd(a.s.tile_sum + v, n);
+    });
+    __syncthreads();
+    if (threadIdx.x < NEAR && near_sum[threadIdx.x]) atomicAdd(a.s.tile_sum + n0 + threadIdx.x, near_sum[threadIdx.x]);
+}
+// the blanked particles of a hash block, and of its group of blocks
+__device__ __forceinline__ void note_blanked(const StepArgs &a, int bid, int nb) {
+    a.s.blank_block[bid] = nb;
+    if (nb) atomicAdd(a.s.blank_group + bid / BLANK_GROUP, nb);
+}
+
 __global__ void kb_clock(BatchTable T, int record_mode);
 __global__ void kb_hash(BatchTable T);
-__global__ void kb_scan_reduce(BatchTable T);
-__global__ void kb_scan_top(BatchTable T);
-__global__ void kb_scan_down(BatchTable T);
+__global__ void kb_scan(BatchTable T);
 __global__ void kb_scatter(BatchTable T);
-__global__ void kb_cell_fixup(BatchTable T);
 cudaError_t launch_gather_predict_batch(const BatchTable &T, bool precision, int blocks, cudaStream_t s);
 __global__ void kb_finalize(BatchTable T);
 __global__ void kb_force_final(BatchTable T);
@@ -173,9 +210,7 @@ cudaError_t launch_interact_batch(const BatchTable &T, bool cspm, int conduction
 
 // the sort kernels on arguments passed by value, for the allocation-free
 // cell-list build (mfree_static.cu)
-__global__ void k_scan_reduce(StepArgs a);
-__global__ void k_scan_top(StepArgs a, int num_tiles, int num_hash_blocks);
-__global__ void k_scan_down(StepArgs a);
+__global__ void k_scan(StepArgs a);
 __global__ void k_scatter(StepArgs a);
 __global__ void k_cell_fixup(StepArgs a);
 

@@ -12,10 +12,12 @@
 //   init, predict                           leap_frog.cu:30-70
 //   do_material_eos, do_corrector_artificial_stress  actions_gpu.cu:40-132
 //
-// The sort is a stable counting sort: an atomic histogram of cell ids, an
-// exclusive scan (which is also the cell-range table the pair loop reads),
-// an atomic scatter and a per-cell fix-up that orders each cell's entries by
-// their previous index.  The result equals thrust's stable sort_by_key of
+// The sort is a stable counting sort: an atomic histogram of cell ids (and of
+// the scan's tiles), an exclusive scan (which is also the cell-range table the
+// pair loop reads), an atomic scatter, and a gather that takes each entry to
+// its rank by previous index within its cell.  Four kernels: for small scenes
+// the launches are what the sort costs (~3.5 us each; separate reduction, scan
+// of the tile sums and per-cell fix-up made it seven).  The result equals thrust's stable sort_by_key of
 // (cell id, 0..n-1): cells ascending, previous order inside a cell, blanked
 // particles (cell id INT_MAX in the reference) last in previous order.
 // N stays on the device: no host round trip per step.
@@ -133,22 +135,9 @@ __device__ __forceinline__ void hash_body(const StepArgs &a, int bid) {
         if (key < unsigned(P.num_cell)) counted = key;
         else blank = 1;
     }
-    // the cell counts: particles come in last step's sorted order, so a
-    // warp's keys run in stretches of one cell; the first lane of each
-    // stretch adds its length (about 14 atomics a warp instead of 32)
-    {
-        const int lane = threadIdx.x & 31;
-        const unsigned prev = __shfl_up_sync(0xffffffffu, counted, 1);
-        const bool start = lane == 0 || prev != counted;
-        const unsigned starts = __ballot_sync(0xffffffffu, start);
-        if (start && counted != 0xffffffffu) {
-            const unsigned after = starts & ~((2u << lane) - 1u);
-            const int end = after ? __ffs(after) - 1 : 32;
-            atomicAdd(&a.s.count[counted], end - lane);
-        }
-    }
+    count_cells(a, counted);
     int nb = __syncthreads_count(blank);
-    if (threadIdx.x == 0) a.s.blank_block[bid] = nb;
+    if (threadIdx.x == 0) note_blanked(a, bid, nb);
 }
 __global__ void __launch_bounds__(HASH_BLOCK) kb_hash(BatchTable T) {
     run_batched(T, T.pblk, [](const StepArgs &a, int b) { hash_body(a, b); });
@@ -182,103 +171,84 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &
     return pre + x - v;
 }
 
-__device__ __forceinline__ void scan_reduce_body(const StepArgs &a, int bid) {
+// Each block sums the tiles before its own (1,734 at most on the 4.1M-particle
+// scene: seven loads a thread), so the tile sums need no scan of their own.
+__device__ __forceinline__ void scan_body(const StepArgs &a, int bid) {
     __shared__ int ws[32];
     const int nc = a.p.num_cell;
-    const int base = bid * SCAN_TILE;
-    int s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) {
-        int c = base + threadIdx.x + k * SCAN_THREADS;
-        if (c < nc) s += a.s.count[c];
-    }
-    int total;
-    block_exclusive_scan(s, ws, total);
-    if (threadIdx.x == 0) a.s.tile_sum[bid] = total;
-}
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(StepArgs a) { scan_reduce_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(SCAN_THREADS) kb_scan_reduce(BatchTable T) {
-    run_batched(T, T.stile, [](const StepArgs &a, int b) { scan_reduce_body(a, b); });
-}
-
-// one block: exclusive scans of the tile sums and of the blanked-per-block counts
-__device__ __forceinline__ void scan_top_body(const StepArgs &a, int num_tiles, int num_hash_blocks) {
-    __shared__ int ws[32];
-    __shared__ int carry;
-    for (int pass = 0; pass < 2; pass++) {
-        int *arr = pass == 0 ? a.s.tile_sum : a.s.blank_block;
-        const int n = pass == 0 ? num_tiles : num_hash_blocks;
-        if (threadIdx.x == 0) carry = 0;
-        __syncthreads();
-        for (int b0 = 0; b0 < n; b0 += 1024) {
-            int idx = b0 + threadIdx.x;
-            int v = idx < n ? arr[idx] : 0;
-            int total;
-            int ex = block_exclusive_scan(v, ws, total);
-            int c0 = carry;
-            if (idx < n) arr[idx] = c0 + ex;
-            __syncthreads();
-            if (threadIdx.x == 0) carry = c0 + total;
-            __syncthreads();
-        }
-        if (pass == 0 && threadIdx.x == 0) a.clk->n_active = carry;
-        __syncthreads();
-    }
-}
-__global__ void __launch_bounds__(1024) k_scan_top(StepArgs a, int num_tiles, int num_hash_blocks) {
-    scan_top_body(a, num_tiles, num_hash_blocks);
-}
-// one block per scene
-__global__ void __launch_bounds__(1024) kb_scan_top(BatchTable T) {
-    __shared__ StepArgs sa;
-    load_scene_args(sa, T, blockIdx.x);
-    __syncthreads();
-    const int tiles = (sa.p.num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE;
-    const int hb = (sa.p.n_init + HASH_BLOCK - 1) / HASH_BLOCK;
-    scan_top_body(sa, tiles, hb);
-}
-
-__device__ __forceinline__ void scan_down_body(const StepArgs &a, int bid) {
-    __shared__ int ws[32];
-    const int nc = a.p.num_cell;
+    int total, before = 0;
+    for (int t = threadIdx.x; t < bid; t += SCAN_THREADS) before += a.s.tile_sum[t];
+    block_exclusive_scan(before, ws, total);
+    const int start = total;
     const int base = bid * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int s = 0;
+    // (the counters and the first table start on 16 bytes, or are read and written one by one)
+    const bool vec = base + SCAN_ITEMS <= nc && ((size_t(a.s.count) | size_t(a.s.first)) & 15) == 0;
+    static_assert(SCAN_ITEMS == 8, "two vectors a thread");
+    if (vec) {
+        const int4 x = reinterpret_cast<const int4 *>(a.s.count + base)[0],
+                   y = reinterpret_cast<const int4 *>(a.s.count + base)[1];
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    } else {
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) {
-        int c = base + k;
-        v[k] = c < nc ? a.s.count[c] : 0;
-        s += v[k];
+        for (int k = 0; k < SCAN_ITEMS; k++) v[k] = base + k < nc ? a.s.count[base + k] : 0;
     }
-    int total;
-    int ex = block_exclusive_scan(s, ws, total) + a.s.tile_sum[bid];
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) {
-        int c = base + k;
-        if (c <= nc) a.s.first[c] = ex;  // first[nc] = N
-        ex += v[k];
+    for (int k = 0; k < SCAN_ITEMS; k++) s += v[k];
+    int ex = block_exclusive_scan(s, ws, total) + start;
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; k++) {  // v becomes the exclusive scan
+        const int n = v[k];
+        v[k] = ex;
+        ex += n;
+    }
+    if (vec) {
+        int4 *f = reinterpret_cast<int4 *>(a.s.first + base);
+        f[0] = make_int4(v[0], v[1], v[2], v[3]);
+        f[1] = make_int4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            if (base + k > nc) break;
+            a.s.first[base + k] = v[k];
+            if (base + k == nc) a.clk->n_active = v[k];  // first[nc] = N
+        }
     }
 }
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(StepArgs a) { scan_down_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(SCAN_THREADS) kb_scan_down(BatchTable T) {
-    run_batched(T, T.stile, [](const StepArgs &a, int b) { scan_down_body(a, b); });
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan(StepArgs a) { scan_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(SCAN_THREADS) kb_scan(BatchTable T) {
+    run_batched(T, T.stile, [](const StepArgs &a, int b) { scan_body(a, b); });
 }
 
 // ---------------------------------------------------------- the scatter --
-__device__ __forceinline__ void scatter_body(const StepArgs &a, int bid) {
+// out: sorted position -> previous position, a cell's entries in no order yet
+__device__ __forceinline__ void scatter_body(const StepArgs &a, int bid, int *out) {
     __shared__ int ws[32];
     const Params &P = a.p;
+    {   // the tile sums are done with: zero for the next step
+        const int tiles = (P.num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE, nb = (P.n_init + HASH_BLOCK - 1) / HASH_BLOCK;
+        for (int t = bid * HASH_BLOCK + threadIdx.x; t < tiles; t += nb * HASH_BLOCK) a.s.tile_sum[t] = 0;
+    }
     const int i = bid * HASH_BLOCK + threadIdx.x;
     const int N = a.clk->n_active;
     unsigned key = i < P.n_init ? a.s.key[i] : 0u;
     int blank = (i < P.n_init && key >= unsigned(P.num_cell)) ? 1 : 0;
-    int total;
-    int rank = block_exclusive_scan(blank, ws, total);
+    int total, rank = 0;
+    if (N < P.n_init) {  // blanked particles: those of the groups and blocks before this one come first
+        const int g = bid / BLANK_GROUP;
+        int before = 0;
+        for (int t = threadIdx.x; t < g; t += HASH_BLOCK) before += a.s.blank_group[t];
+        for (int t = g * BLANK_GROUP + threadIdx.x; t < bid; t += HASH_BLOCK) before += a.s.blank_block[t];
+        block_exclusive_scan(before, ws, total);
+        const int start = total;
+        rank = start + block_exclusive_scan(blank, ws, total);
+    }
     // one atomic per stretch of equal keys in the warp (the hash kernel's
     // stretches): its first lane takes the stretch's length off the cell's
     // count (which leaves count[] zero for the next step) and the stretch
-    // fills its slots in lane order, so it arrives in increasing index order
-    // and the per-cell fix-up below has little to move
+    // fills its slots in lane order
     const int lane = threadIdx.x & 31;
     const unsigned counted = (i < P.n_init && !blank) ? key : 0xffffffffu;
     const unsigned prev = __shfl_up_sync(0xffffffffu, counted, 1);
@@ -294,18 +264,16 @@ __device__ __forceinline__ void scatter_body(const StepArgs &a, int bid) {
     if (i >= P.n_init) return;
     if (!blank) {
         const int d = a.s.first[key] + old - (end - head) + (lane - head);
-        if (bounds_ok(a.clk, d, P.n_init)) a.s.perm[d] = i;
+        if (bounds_ok(a.clk, d, P.n_init)) out[d] = i;
     } else {
-        const int d = N + a.s.blank_block[bid] + rank;
-        if (bounds_ok(a.clk, d, P.n_init)) a.s.perm[d] = i;
+        const int d = N + rank;
+        if (bounds_ok(a.clk, d, P.n_init)) out[d] = i;
     }
 }
-__global__ void __launch_bounds__(HASH_BLOCK) k_scatter(StepArgs a) { scatter_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(HASH_BLOCK) kb_scatter(BatchTable T) {
-    run_batched(T, T.pblk, [](const StepArgs &a, int b) { scatter_body(a, b); });
-}
+__global__ void __launch_bounds__(HASH_BLOCK) k_scatter(StepArgs a) { scatter_body(a, blockIdx.x, a.s.perm); }
 
-// order each cell's entries by previous index (stable within the cell)
+// order each cell's entries by previous index (stable within the cell), in
+// place; the step's gather ranks them instead
 __device__ __forceinline__ void cell_fixup_body(const StepArgs &a, int bid) {
     const int c = bid * 256 + threadIdx.x;
     if (c >= a.p.num_cell) return;
@@ -390,28 +358,45 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
     if (n > 0) flush();
 }
 
-// blocks past the cell blocks of every scene build the tile list (the cell
-// starts are final once the scatter has run)
-__global__ void __launch_bounds__(256) kb_cell_fixup(BatchTable T) {
-    const int nb = T.cblk[T.nscenes];
-    if (int(blockIdx.x) >= nb) {
-        tile_list_body(T, (int(blockIdx.x) - nb) * 8 + int(threadIdx.x >> 5), int(threadIdx.x & 31));
+// the first blocks build the tile list (the cell starts are final once the scan
+// has run), the others scatter
+__global__ void __launch_bounds__(HASH_BLOCK) kb_scatter(BatchTable T) {
+    const int tb = (T.ibun[T.nscenes] + 7) / 8, b = int(blockIdx.x) - tb;
+    if (b < 0) {
+        tile_list_body(T, int(blockIdx.x) * 8 + int(threadIdx.x >> 5), int(threadIdx.x & 31));
         return;
     }
-    run_batched(T, T.cblk, [](const StepArgs &a, int b) { cell_fixup_body(a, b); });
+    const int s = find_scene(T.pblk, T.nscenes, b);
+    const StepArgs &a = scene_args(T, s);
+    scatter_body(a, b - T.pblk[s], a.s.perm_raw);
 }
 
 // --------------------------------------------- gather + predictor + EOS --
 template <bool PREC> __device__ __forceinline__ void gather_predict_body(const StepArgs &a, int bid) {
     const Params &P = a.p;
-    const int i = bid * 256 + threadIdx.x;
+    int i = bid * 256 + threadIdx.x;
+    {   // the groups' blanked counts are done with: zero for the next step
+        const int groups = (P.n_init + HASH_BLOCK * BLANK_GROUP - 1) / (HASH_BLOCK * BLANK_GROUP);
+        if (i < groups) a.s.blank_group[i] = 0;
+    }
     if (i >= P.n_init) return;
     const int N = a.clk->n_active;
-    int src = a.s.perm[i];
+    int src = a.s.perm_raw[i];
     if (src < 0 || src >= P.n_init) {  // cannot happen for a consistent sort; never read out of bounds
         atomicAdd(&a.clk->out_of_grid, 1ull << 32);
         src = i;
     }
+    const unsigned key = a.s.key[src];
+    if (i < N && key < unsigned(P.num_cell)) {
+        // the entry's place in its cell: its rank by previous index (a cell
+        // holds about two; the scatter leaves them in no order)
+        const int c0 = a.s.first[key], c1 = a.s.first[key + 1];
+        if (c1 - c0 > 1 && bounds_ok(a.clk, c0, P.n_init) && bounds_ok(a.clk, c1 - 1, P.n_init)) {
+            i = c0;
+            for (int k = c0; k < c1; k++) i += a.s.perm_raw[k] < src ? 1 : 0;
+        }
+    }
+    a.s.perm[i] = src;
     const State &A = a.a, &B = a.b;
     float4 pos = A.pos4[src], vel = A.vel4[src], sa = A.sa4[src], sb = A.sb4[src];
     float4 da = A.da4[src], dv = A.dv4[src], dsa = A.dsa4[src], dsb = A.dsb4[src];
@@ -426,7 +411,7 @@ template <bool PREC> __device__ __forceinline__ void gather_predict_body(const S
         B.lo4[i] = lo;
         B.lo4b[i] = lob;
     }
-    a.s.key_sorted[i] = a.s.key[src];
+    a.s.key_sorted[i] = key;
     if (i >= N) return;  // blanked: frozen
     const float h2 = 0.5f * P.dt;
     HalfStep hs = half_step<PREC>(h2, pos, vel, sa, sb, da, dv, dsa, dsb, lo, lob);

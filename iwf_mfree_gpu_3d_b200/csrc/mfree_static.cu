@@ -16,6 +16,7 @@
 // are cleared at the start of each call, and calls that overlap on the GPU
 // (different streams, or different host threads on one device) race on it.
 #include <atomic>
+#include <cstddef>
 #include <cstring>
 #include <string>
 
@@ -29,12 +30,14 @@ namespace {
 constexpr int MAX_N = MFREE_STATIC_MAX_PARTICLES;
 constexpr int MAX_CELLS = MFREE_STATIC_MAX_CELLS;
 constexpr int MAX_TILES = (MAX_CELLS + 1 + SCAN_TILE - 1) / SCAN_TILE + 1;
+constexpr int MAX_GROUPS = (MAX_N + HASH_BLOCK * BLANK_GROUP - 1) / (HASH_BLOCK * BLANK_GROUP);
 constexpr int MAX_HASH_BLOCKS = (MAX_N + HASH_BLOCK - 1) / HASH_BLOCK + 1;
 
 struct StaticScratch {
     unsigned key[MAX_N];
-    int count[MAX_CELLS + 1];
-    int tile_sum[MAX_TILES];
+    int tile_sum[MAX_TILES];        // cleared at the start of each call, with the group counts and
+    int blank_group[MAX_GROUPS];    // the cells in use of the counters behind them
+    alignas(16) int count[MAX_CELLS + 1];
     int blank_block[MAX_HASH_BLOCKS];
     DevClock clk;
 };
@@ -62,6 +65,7 @@ __global__ void __launch_bounds__(HASH_BLOCK) k_hash_positions(StepArgs a, const
     const Params &P = a.p;
     const int i = blockIdx.x * HASH_BLOCK + threadIdx.x;
     int blank = 0;
+    unsigned counted = 0xffffffffu;  // the cell this position is counted in (none: all ones)
     if (i < P.n_init) {
         const float4 p = pos[i];
         unsigned key = unsigned(P.num_cell);
@@ -72,11 +76,12 @@ __global__ void __launch_bounds__(HASH_BLOCK) k_hash_positions(StepArgs a, const
         if (finite && ix >= 0 && ix < P.gnx && iy >= 0 && iy < P.gny && iz >= 0 && iz < P.gnz)
             key = unsigned((ix * P.gny + iy) * P.gnz + iz);
         a.s.key[i] = key;
-        if (key < unsigned(P.num_cell)) atomicAdd(&a.s.count[key], 1);
+        if (key < unsigned(P.num_cell)) counted = key;
         else blank = 1;
     }
+    count_cells(a, counted);
     const int nb = __syncthreads_count(blank);
-    if (threadIdx.x == 0) a.s.blank_block[blockIdx.x] = nb;
+    if (threadIdx.x == 0) note_blanked(a, blockIdx.x, nb);
 }
 
 int sfail(int code, const std::string &m) {
@@ -127,16 +132,16 @@ extern "C" int mfree_cell_list_static(const float *pos4, int n, const float bbmi
     a.s.first = cell_first;
     a.s.tile_sum = S->tile_sum;
     a.s.blank_block = S->blank_block;
+    a.s.blank_group = S->blank_group;
     a.s.perm = perm;
     a.clk = &S->clk;
     const int hb = (n + HASH_BLOCK - 1) / HASH_BLOCK;
     const int tiles = int((ncell + 1 + SCAN_TILE - 1) / SCAN_TILE);
-    e = cudaMemsetAsync(S->count, 0, sizeof(int) * size_t(ncell + 1), s);  // the last call may have left counts
+    // the last call may have left counts
+    e = cudaMemsetAsync(S->tile_sum, 0, offsetof(StaticScratch, count) - offsetof(StaticScratch, tile_sum) + sizeof(int) * size_t(ncell + 1), s);
     if (e != cudaSuccess) return sfail(MFREE_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
     k_hash_positions<<<hb, HASH_BLOCK, 0, s>>>(a, (const float4 *)pos4, bbmin[0], bbmin[1], bbmin[2]);
-    k_scan_reduce<<<tiles, SCAN_THREADS, 0, s>>>(a);
-    k_scan_top<<<1, 1024, 0, s>>>(a, tiles, hb);
-    k_scan_down<<<tiles, SCAN_THREADS, 0, s>>>(a);
+    k_scan<<<tiles, SCAN_THREADS, 0, s>>>(a);
     k_scatter<<<hb, HASH_BLOCK, 0, s>>>(a);
     k_cell_fixup<<<int((ncell + 255) / 256), 256, 0, s>>>(a);
     e = cudaGetLastError();
