@@ -166,15 +166,20 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     const BatchTable &T = b->T;
     cudaStream_t s = b->stream;
     const int n = T.nscenes;
-    kb_clock<<<(n + 127) / 128, 128, 0, s>>>(T, record_mode);
-    kb_hash<<<b->tot_pblk, HASH_BLOCK, 0, s>>>(T);
-    kb_scan<<<b->tot_stile, SCAN_THREADS, 0, s>>>(T);
-    kb_scatter<<<b->tot_pblk + (b->tot_ibun + 7) / 8, HASH_BLOCK, 0, s>>>(T);
-    cudaError_t e = launch_gather_predict_batch(T, b->prec, b->tot_pblk, s);
-    if (e == cudaSuccess) e = launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s);
+    cudaError_t e = cudaSuccess;
+    auto run = [&](auto &&launch) {
+        if (e == cudaSuccess) e = launch();
+    };
+    run([&] { return launch_after(kb_clock, (n + 127) / 128, 128, 0, s, T, record_mode); });
+    run([&] { return launch_after(kb_hash, b->tot_pblk, HASH_BLOCK, 0, s, T); });
+    run([&] { return launch_after(kb_scan, b->tot_stile, SCAN_THREADS, 0, s, T); });
+    run([&] { return launch_after(kb_scatter, b->tot_pblk + (b->tot_ibun + 7) / 8, HASH_BLOCK, 0, s, T); });
+    run([&] { return launch_gather_predict_batch(T, b->prec, b->tot_pblk, s); });
+    run([&] { return launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s); });
+    run([&] { return launch_after(kb_finalize, b->tot_pblk, FIN_BLOCK, 0, s, T); });
+    if (record_mode == 1 || (record_mode == 2 && b->table_record_every > 0))
+        run([&] { return launch_after(kb_force_final, n, 256, 0, s, T); });
     if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("batched step launch: ") + cudaGetErrorString(e));
-    kb_finalize<<<b->tot_pblk, FIN_BLOCK, 0, s>>>(T);
-    if (record_mode == 1 || (record_mode == 2 && b->table_record_every > 0)) kb_force_final<<<n, 256, 0, s>>>(T);
     CUDA_TRY(cudaGetLastError());
     return MFREE_OK;
 }

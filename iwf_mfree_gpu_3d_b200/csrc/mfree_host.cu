@@ -363,6 +363,7 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     const int nb = (c->n_init + 255) / 256;
     cudaError_t le = cudaSuccess;
     auto run = [&](int id, auto &&launch) {
+        if (le != cudaSuccess) return;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (timed) {
             e0 = pooled_event(c);
@@ -376,18 +377,17 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
             c->tev.push_back({id, {e0, e1}});
         }
     };
-    run(0, [&] { kb_clock<<<1, 32, 0, s>>>(T, record_mode); });
-    run(1, [&] { kb_hash<<<hb, HASH_BLOCK, 0, s>>>(T); });
-    run(4, [&] { kb_scan<<<tiles, SCAN_THREADS, 0, s>>>(T); });
-    run(5, [&] { kb_scatter<<<hb + (c->nbun + 7) / 8, HASH_BLOCK, 0, s>>>(T); });
+    run(0, [&] { le = launch_after(kb_clock, 1, 32, 0, s, T, record_mode); });
+    run(1, [&] { le = launch_after(kb_hash, hb, HASH_BLOCK, 0, s, T); });
+    run(4, [&] { le = launch_after(kb_scan, tiles, SCAN_THREADS, 0, s, T); });
+    run(5, [&] { le = launch_after(kb_scatter, hb + (c->nbun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run(7, [&] { le = launch_gather_predict_batch(T, P.precision != 0, nb, s); });
-    if (le == cudaSuccess)
-        run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
-    if (le != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(le));
-    run(9, [&] { kb_finalize<<<finalize_blocks(c->n_init), FIN_BLOCK, 0, s>>>(T); });
+    run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
+    run(9, [&] { le = launch_after(kb_finalize, finalize_blocks(c->n_init), FIN_BLOCK, 0, s, T); });
     // (a step that cannot record needs no sum of the recorded forces)
     if (!c->tools.empty() && (record_mode == 1 || (record_mode == 2 && record_every > 0)))
-        run(10, [&] { kb_force_final<<<1, 256, 0, s>>>(T); });
+        run(10, [&] { le = launch_after(kb_force_final, 1, 256, 0, s, T); });
+    if (le != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(le));
     CUDA_TRY(cudaGetLastError());
     return MFREE_OK;
 }

@@ -581,6 +581,7 @@ constexpr long long WAIT_CYCLES = 1ll << 30;  // bound of a staging wait (~0.5 s
 // a tile's tables, built by the producer warp one tile ahead (two buffers)
 struct TileTab {
     int cs[NHC][CSROW];   // record index (staged) or sorted index of the cell starts of each halo column
+    int shift[NHC];       // record index minus sorted index of each halo column (staged)
     int trec[NTC];        // record index of each target column's first target
     int tsrt[NTC];        // its sorted index
     int tpref[NTC + 1];   // targets before the column
@@ -591,7 +592,7 @@ struct TileTab {
 struct BlockSmem {
     TileTab tab[2];
     unsigned long long bar;
-    int fail, list_n;
+    int fail;
 };
 __host__ __device__ constexpr size_t round128(size_t b) { return (b + 127) / 128 * 128; }
 // shared memory: the tables, the arguments of two scenes, the queues, the staged records
@@ -901,13 +902,15 @@ __device__ __forceinline__ void produce(const BatchTable &T, BlockSmem &sm, Step
     int slot_scene[2] = {-1, -1};  // scenes whose arguments the two slots hold
     int slot = 0;
     int2 e = make_int2(0, -1);
+    // the first entry is the block's own, the others are claimed
+    const int list_n = *T.tile_count;
+    if (lane == 0 && int(blockIdx.x) < list_n) e = T.tile_list[blockIdx.x];
     auto claim = [&] {
         if (lane == 0) {
-            const int k = atomicAdd(T.tile_next, 1);
-            e = k < sm.list_n ? T.tile_list[k] : make_int2(0, -1);
+            const int k = atomicAdd(T.tile_next, 1) + int(gridDim.x);
+            e = k < list_n ? T.tile_list[k] : make_int2(0, -1);
         }
     };
-    claim();
 #pragma unroll 1
     for (int n = 0;; n++) {
         const int t = __shfl_sync(0xffffffffu, e.x, 0), sd = __shfl_sync(0xffffffffu, e.y, 0);
@@ -938,8 +941,8 @@ __device__ __forceinline__ void produce(const BatchTable &T, BlockSmem &sm, Step
         // halo cell starts (sorted indices), each lane's loads in flight together
         constexpr int NCS = NHC * CSROW / 32;
         static_assert(NHC * CSROW % 32 == 0, "whole warps of cell starts");
+        int csv[NCS];
         {
-            int csv[NCS];
 #pragma unroll
             for (int r = 0; r < NCS; r++) {
                 const int x = lane + r * 32;
@@ -947,7 +950,7 @@ __device__ __forceinline__ void produce(const BatchTable &T, BlockSmem &sm, Step
                 const int cx = G.X0 - 2 + c / HY, cy = G.Y0 - 2 + c % HY;
                 csv[r] = 0;
                 if (k < G.nzr && cx >= 0 && cx < nx && cy >= 0 && cy < ny) {
-                    const long long fi = (long long)(cx * ny + cy) * nz + G.zl + k;
+                    const int fi = (cx * ny + cy) * nz + G.zl + k;
                     if (bounds_ok(a.clk, fi, (long long)P.num_cell + 1)) csv[r] = first[fi];
                 }
             }
@@ -997,12 +1000,14 @@ __device__ __forceinline__ void produce(const BatchTable &T, BlockSmem &sm, Step
         if (lane < NTC) tab.tpref[lane] = ti - len;
         if (lane == 31) tab.tpref[NTC] = ti;
         __syncwarp();
-        if (staged) {  // the cell starts as record indices
+        if (staged) {  // the cell starts as record indices: every lane shifts those it holds
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const int c = 2 * lane + k, d = ho[k] - hs[k];
-                if (hl[k] > 0)
-                    for (int q = 0; q < G.nzr; q++) tab.cs[c][q] += d;
+            for (int k = 0; k < 2; k++) tab.shift[2 * lane + k] = hl[k] > 0 ? ho[k] - hs[k] : int(0x80000000);
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < NCS; r++) {
+                const int x = lane + r * 32, d = tab.shift[x / CSROW];
+                if (d != int(0x80000000)) (&tab.cs[0][0])[x] = csv[r] + d;
             }
         }
         __syncwarp();
@@ -1075,8 +1080,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) kb_interact(BatchTable T) {
     unsigned short *queue = reinterpret_cast<unsigned short *>(dyn + QUEUE_OFFSET);
     float4 *sarr = reinterpret_cast<float4 *>(dyn + REC_OFFSET);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    begin_after();
     if (threadIdx.x == 0) {
-        sm.list_n = *T.tile_count;
         sm.fail = 0;
         mbar_init(&sm.bar, 1);
     }
@@ -1150,8 +1155,7 @@ template <bool CSPM, int COND, bool PREC> struct Variant {
         auto kern = kb_interact<CSPM, COND, PREC>;
         if (grid <= 0)  // prepare only: raise the shared-memory limit (outside any graph capture)
             return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
-        kern<<<grid, NTHREADS, SMEM_LIMIT, s>>>(T);
-        return cudaGetLastError();
+        return launch_after(kern, grid, NTHREADS, SMEM_LIMIT, s, T);
     }
 };
 

@@ -129,6 +129,35 @@ inline long long max_tiles(const Params &P) {
     return (long long)num_bundles(P) * (P.gnz / P.tile_z + 2) + 2ll * P.n_init / P.tile_cap + 2;
 }
 
+// Programmatic dependent launch: a step's kernels are launched while the one
+// before still runs (launch_after), so that launch latency and block start-up
+// are hidden; each begins with begin_after, which waits until the kernel before
+// has completed and its writes are visible, and only then lets the next one
+// start.  So a kernel never overlaps the work of another, only its launch.
+// Inside a stream capture the launches are plain: in a graph the programmatic
+// edges cost more than they hide (8,000 particles, a step: eager 142 -> 129 us,
+// graph 74.6 -> 76.3 us).
+__device__ __forceinline__ void begin_after() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... K, class... A>
+inline cudaError_t launch_after(void (*kern)(K...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(unsigned(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaError_t e = cudaStreamIsCapturing(s, &cap)) return e;
+    cfg.attrs = &at;
+    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, K(args)...);
+}
+
 // scene of block x: the last s with prefix[s] <= x (prefix has nscenes + 1 entries)
 __device__ __forceinline__ int find_scene(const int *__restrict__ prefix, int nscenes, int x) {
     int lo = 0, hi = nscenes - 1;

@@ -67,6 +67,7 @@ __device__ __forceinline__ void clock_body(const StepArgs &a, int record_mode) {
 
 // one thread per scene; thread 0 also resets the batch's pair-kernel queue
 __global__ void kb_clock(BatchTable T, int record_mode) {
+    begin_after();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) {
         *T.tile_next = 0;
@@ -140,6 +141,7 @@ __device__ __forceinline__ void hash_body(const StepArgs &a, int bid) {
     if (threadIdx.x == 0) note_blanked(a, bid, nb);
 }
 __global__ void __launch_bounds__(HASH_BLOCK) kb_hash(BatchTable T) {
+    begin_after();
     run_batched(T, T.pblk, [](const StepArgs &a, int b) { hash_body(a, b); });
 }
 
@@ -217,8 +219,12 @@ __device__ __forceinline__ void scan_body(const StepArgs &a, int bid) {
         }
     }
 }
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan(StepArgs a) { scan_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan(StepArgs a) {
+    begin_after();
+    scan_body(a, blockIdx.x);
+}
 __global__ void __launch_bounds__(SCAN_THREADS) kb_scan(BatchTable T) {
+    begin_after();
     run_batched(T, T.stile, [](const StepArgs &a, int b) { scan_body(a, b); });
 }
 
@@ -270,7 +276,10 @@ __device__ __forceinline__ void scatter_body(const StepArgs &a, int bid, int *ou
         if (bounds_ok(a.clk, d, P.n_init)) out[d] = i;
     }
 }
-__global__ void __launch_bounds__(HASH_BLOCK) k_scatter(StepArgs a) { scatter_body(a, blockIdx.x, a.s.perm); }
+__global__ void __launch_bounds__(HASH_BLOCK) k_scatter(StepArgs a) {
+    begin_after();
+    scatter_body(a, blockIdx.x, a.s.perm);
+}
 
 // order each cell's entries by previous index (stable within the cell), in
 // place; the step's gather ranks them instead
@@ -291,7 +300,10 @@ __device__ __forceinline__ void cell_fixup_body(const StepArgs &a, int bid) {
         p[m + 1] = v;
     }
 }
-__global__ void __launch_bounds__(256) k_cell_fixup(StepArgs a) { cell_fixup_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(256) k_cell_fixup(StepArgs a) {
+    begin_after();
+    cell_fixup_body(a, blockIdx.x);
+}
 
 // The pair kernel's list of non-empty tiles: one warp per bundle of every
 // scene.  Lane k holds the targets below level base + k of the bundle, so a
@@ -361,6 +373,7 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
 // the first blocks build the tile list (the cell starts are final once the scan
 // has run), the others scatter
 __global__ void __launch_bounds__(HASH_BLOCK) kb_scatter(BatchTable T) {
+    begin_after();
     const int tb = (T.ibun[T.nscenes] + 7) / 8, b = int(blockIdx.x) - tb;
     if (b < 0) {
         tile_list_body(T, int(blockIdx.x) * 8 + int(threadIdx.x >> 5), int(threadIdx.x & 31));
@@ -447,6 +460,7 @@ template <bool PREC> __device__ __forceinline__ void gather_predict_body(const S
     if (P.diagnostics) a.s.pos_half[i] = make_float4(hs.x, hs.y, hs.z, 0.f);
 }
 template <bool PREC> __global__ void __launch_bounds__(256) kb_gather_predict(BatchTable T) {
+    begin_after();
     run_batched(T, T.pblk, [](const StepArgs &a, int b) { gather_predict_body<PREC>(a, b); });
 }
 
@@ -484,9 +498,7 @@ cudaError_t launch_init_state(int n, const float4 *pos, const float4 *vel, const
 }
 
 cudaError_t launch_gather_predict_batch(const BatchTable &T, bool precision, int blocks, cudaStream_t s) {
-    if (precision) kb_gather_predict<true><<<blocks, 256, 0, s>>>(T);
-    else kb_gather_predict<false><<<blocks, 256, 0, s>>>(T);
-    return cudaGetLastError();
+    return launch_after(precision ? kb_gather_predict<true> : kb_gather_predict<false>, blocks, 256, 0, s, T);
 }
 
 }  // namespace mfree

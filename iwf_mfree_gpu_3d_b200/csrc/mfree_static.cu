@@ -62,6 +62,7 @@ std::atomic<StaticScratch *> g_scratch_addr[MAX_DEVICES];
 // lower corner still falls in cell 0 of that axis.
 __global__ void __launch_bounds__(HASH_BLOCK) k_hash_positions(StepArgs a, const float4 *pos, float bx, float by,
                                                                float bz) {
+    begin_after();
     const Params &P = a.p;
     const int i = blockIdx.x * HASH_BLOCK + threadIdx.x;
     int blank = 0;
@@ -140,11 +141,11 @@ extern "C" int mfree_cell_list_static(const float *pos4, int n, const float bbmi
     // the last call may have left counts
     e = cudaMemsetAsync(S->tile_sum, 0, offsetof(StaticScratch, count) - offsetof(StaticScratch, tile_sum) + sizeof(int) * size_t(ncell + 1), s);
     if (e != cudaSuccess) return sfail(MFREE_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-    k_hash_positions<<<hb, HASH_BLOCK, 0, s>>>(a, (const float4 *)pos4, bbmin[0], bbmin[1], bbmin[2]);
-    k_scan<<<tiles, SCAN_THREADS, 0, s>>>(a);
-    k_scatter<<<hb, HASH_BLOCK, 0, s>>>(a);
-    k_cell_fixup<<<int((ncell + 255) / 256), 256, 0, s>>>(a);
-    e = cudaGetLastError();
+    e = launch_after(k_hash_positions, hb, HASH_BLOCK, 0, s, a, (const float4 *)pos4, bbmin[0], bbmin[1], bbmin[2]);
+    if (e == cudaSuccess) e = launch_after(k_scan, tiles, SCAN_THREADS, 0, s, a);
+    if (e == cudaSuccess) e = launch_after(k_scatter, hb, HASH_BLOCK, 0, s, a);
+    if (e == cudaSuccess) e = launch_after(k_cell_fixup, int((ncell + 255) / 256), 256, 0, s, a);
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return sfail(MFREE_ERR_CUDA, std::string("cell list kernels: ") + cudaGetErrorString(e));
     return MFREE_OK;
 }
