@@ -23,24 +23,35 @@
 // copies per column, its P records and the interleaved rest (TMA
 // cp.async.bulk, completion counted on an mbarrier, bounded waits).
 //
-// Two lanes serve a target; the 512 compute threads hold up to 256 targets of
-// a tile at once, each from its candidates to its new state without a barrier
-// in between.  The candidate pass walks the 25 stencil columns of the target's
+// Two lanes serve a target; the 480 compute threads hold up to 240 targets of
+// a tile at once, each from its candidates to its new state without a block
+// barrier in between.  The candidate pass walks the 25 stencil columns of the target's
 // cell, the two lanes on alternate records, and puts the in-support neighbours
 // into a queue that the lanes fill from its two ends.  The pair pass runs on
 // the queue only -- the reference evaluates the pair body for every candidate,
 // ~3.5x more work, and candidates outside the support contribute exact zeros
-// there.  One shuffle per sum joins the two lanes, then the first runs the
-// fused rest of the step.  A producer warp builds the next tile's tables
+// there.  Four lanes share a target's queue there; their sums are joined by
+// shuffles, then the first of its two lanes runs the fused rest of the step.  A producer warp builds the next tile's tables
 // while the compute warps work, and issues its copies as soon as they have
 // read the last record of the current tile, so that the copies land while the
 // epilogue runs.
 //
-// The kernel is bound by instruction issue, not by the FP32 pipe or memory:
-// the split follows from the instructions it saves.  Eight lanes a target (an
+// What bounds it: instruction issue (half of the cycles) and shared-memory
+// wavefronts (55 %), with 16 warps an SM -- the registers and the staged halo
+// leave room for no more -- to hide latencies, and 29 % of warp time at the
+// tile's barriers; FP32 pipe 23 %, DRAM 3 % (ncu, 252,000 particles).  The split
+// follows from the instructions it saves: eight lanes a target throughout (an
 // earlier form) spent about 80 instruction slots a candidate on ballots and on
-// walking columns that are about as long as the group is wide, and reduced 25
-// sums over 8 lanes.
+// walking columns that are about as long as the group is wide.  Pair kernel,
+// us, that form -> this one: 1M with CSPM + PSE 1845 -> 1258, 1M with every
+// temperature different 2062 -> 1396, 4.1M with Brookshaw 6646 -> 4575, 252,000
+// 473 -> 323 (eager event times).
+//
+// Tried and slower: 2 or 3 candidates a lane at once (+2 %, +1 %); two queue
+// entries a lane and iteration (+-0 with four lanes); 12 warps with 168 registers
+// and no spills (+3 % at 1M, +8 % at 4.1M; -7 % at 30,000 particles); the
+// epilogue's state prefetched into L2 by the producer warp (+11 %); compute warps
+// polling the mbarrier themselves (+-0).
 #pragma once
 
 #include <type_traits>
@@ -190,7 +201,7 @@ template <bool CSPM, int COND> struct Sums {
     }
     // the sums over the LANES lanes of a group, left in row[0..COUNT) (shared
     // memory): a butterfly that halves the list at every step, so a lane ends
-    // with an eighth of it.  Every lane of the warp calls it.
+    // with a quarter of it.  Every lane of the warp calls it.
     template <int LANES> __device__ __forceinline__ void reduce_to(float *row, int l, bool store) {
         fold();
         constexpr int REST = COUNT % 8 <= 2 ? COUNT % 8 : 0;  // few left over: reduced in full
@@ -200,7 +211,7 @@ template <bool CSPM, int COND> struct Sums {
         for (int k = 0; k < MAIN + 8; k++) a[k] = 0.f;
         int n = 0;
         each([&](float &v) { a[n++] = v; });
-        constexpr int STEPS = LANES == 8 ? 3 : 1;
+        constexpr int STEPS = LANES == 4 ? 2 : 1;
         int base = 0;
 #pragma unroll
         for (int st = 0; st < STEPS; st++) {
@@ -568,6 +579,8 @@ constexpr int CSROW = TILE_Z_MAX + 5;  // cell starts kept per halo column
 constexpr int NHC = HX * HY;           // halo columns
 constexpr int NTC = TX * TY;           // target columns
 constexpr int LPT = 2;                 // lanes per target
+constexpr int PPT = 4;                 // lanes per target in the pair pass
+constexpr int TPR = 32 / PPT;          // targets of a warp at a time there
 constexpr int NCOMP = 480;             // compute threads
 constexpr int NTHREADS = NCOMP + 32;   // and the producer warp: 16 warps, 128 registers a thread
 constexpr int TCAP = NCOMP / LPT;      // targets per pass of a tile
@@ -816,20 +829,21 @@ __device__ __forceinline__ int process_target(const StepArgs &a, const TileTab &
     const int nq = qn + qo;
     const bool queued = nq <= QCAP && max(qn, qo) <= QCAP - CH;
     if (COND == MFREE_COND_PSE) pse += __shfl_xor_sync(0xffffffffu, pse, 1);
-    // ---- pair body over the in-support neighbours: eight lanes a target, four
-    // targets of the warp at a time; lanes 0-3 take the queue's front part,
-    // lanes 4-7 its back part.  Their entries are mostly neighbouring records,
-    // which lie on different banks (with two lanes a target the sixteen targets
-    // of a warp read unrelated records: 12 wavefronts a load instead of ~5).
+    // ---- pair body over the in-support neighbours: four lanes a target, eight
+    // targets of the warp at a time; lanes 0 and 1 take the queue's front part,
+    // lanes 2 and 3 its back part.  A target's entries are mostly neighbouring
+    // records, which lie on different banks, so more lanes a target mean fewer
+    // conflicts, and a longer reduction with more idle lanes at the end: pair
+    // kernel on the 1M step 1288 / 1258 / 1314 us with two / four / eight.
     // A target's sums replace its queue row.
     const int lane = threadIdx.x & 31;
     const PairConst PC{0.25f * P.av_eta * P.av_eta, -0.5f * P.av_alpha, 0.5f * P.av_beta};
     {
-        const int l = lane & 7, back = l >> 2;
+        const int l = lane % PPT, back = l >= PPT / 2, lh = l % (PPT / 2);
         Q *const wrow = qrow - size_t(lane / LPT) * QROW;  // the warp's first row
 #pragma unroll 1
         for (int rd = 0; rd < rounds; rd++) {
-            const int tl = rd * 4 + (lane >> 3), own = tl * LPT;
+            const int tl = rd * TPR + lane / PPT, own = tl * LPT;
             const int n_f = __shfl_sync(0xffffffffu, queued && valid ? qn : 0, own);
             const int n_b = __shfl_sync(0xffffffffu, queued && valid ? qn : 0, own + 1);
             const int sj = __shfl_sync(0xffffffffu, si, own);
@@ -841,27 +855,27 @@ __device__ __forceinline__ int process_target(const StepArgs &a, const TileTab &
             J.art = I.art;
             target_of<CSPM, COND>(RF[sj], X + sj * REC_X, J);
             Q *const row = wrow + tl * QROW;
-            const Q *qe = back ? row + (QCAP - 1) - (l & 3) : row + (l & 3);
-            const int qd = back ? -4 : 4, cnt = back ? n_b : n_f;
+            const Q *qe = back ? row + (QCAP - 1) - lh : row + lh;
+            const int qd = back ? -(PPT / 2) : PPT / 2, cnt = back ? n_b : n_f;
             Sums<CSPM, COND> S;
             S.zero();
             // the next entry's index and position are read ahead
-            int m = l & 3;
+            int m = lh;
             int j = m < cnt ? int(*qe) : sj;
             float4 Pj = RF[j];
-            int jn = m + 4 < cnt ? int(qe[qd]) : j;
+            int jn = m + PPT / 2 < cnt ? int(qe[qd]) : j;
 #pragma unroll 1
-            for (; m < cnt; m += 4) {
+            for (; m < cnt; m += PPT / 2) {
                 const float4 Pc = Pj;
                 const int jc = j;
                 j = jn;
                 Pj = RF[j];
                 qe += qd;
-                jn = m + 8 < cnt ? int(qe[qd]) : j;
+                jn = m + PPT < cnt ? int(qe[qd]) : j;
                 pair_body<CSPM, COND>(PC, J, Pc, X + jc * REC_X, S);
             }
             __syncwarp();
-            S.template reduce_to<8>(reinterpret_cast<float *>(row), l, n_f + n_b > 0);
+            S.template reduce_to<PPT>(reinterpret_cast<float *>(row), l, n_f + n_b > 0);
         }
     }
     __syncwarp();
@@ -1123,12 +1137,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) kb_interact(BatchTable T) {
         for (int t0 = 0;; t0 += TCAP) {
             float res[NRES];
             int i = -1;
-            // targets a warp: its rounds of the pair pass (four targets each) are
+            // targets a warp: its rounds of the pair pass (eight targets each) are
             // what a tile waits for, so few targets are spread over all warps
-            const int rounds = min(32 / LPT / 4, (min(ntg - t0, TCAP) + NCOMP / 8 - 1) / (NCOMP / 8));
-            const int tw = t0 + warp * (4 * rounds);  // the warp's first target
+            const int rounds = min(32 / LPT / TPR, (min(ntg - t0, TCAP) + NCOMP / PPT - 1) / (NCOMP / PPT));
+            const int tw = t0 + warp * (TPR * rounds);  // the warp's first target
             if (tw < min(ntg, t0 + TCAP)) {
-                const int tt = lane / LPT < 4 * rounds ? tw + lane / LPT : ntg;
+                const int tt = lane / LPT < TPR * rounds ? tw + lane / LPT : ntg;
                 if (staged && COND == MFREE_COND_PSE && pse_zero)
                     i = process_target<CSPM, MFREE_COND_NONE, true>(a, tab, queue, sarr, ntg, tt, sl, rounds, res);
                 else if (staged)
