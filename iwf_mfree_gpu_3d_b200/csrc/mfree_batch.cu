@@ -19,6 +19,7 @@
 // data, a scene's results are the same alone and in a batch for the same
 // pair-loop tiling.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <memory>
 #include <string>
@@ -150,6 +151,7 @@ int build_table(mfree_batch *b, int record_every) {
         b->tiles_cap = cap;
     }
     b->T.tile_list = b->d_tiles;
+    b->T.tile_max = int(std::min<long long>(b->tiles_cap, INT_MAX));
     // pageable sources: the call returns once the bytes are staged, so the
     // vectors may go; the device copy stays ordered on the stream
     CUDA_TRY(cudaMemcpyAsync(dargs, args.data(), sizeof(StepArgs) * args.size(), cudaMemcpyHostToDevice, b->stream));

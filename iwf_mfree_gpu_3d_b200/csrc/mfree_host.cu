@@ -344,6 +344,7 @@ int ensure_table(mfree_ctx *c, int record_every) {
     c->T.tile_next = di + 6;
     c->T.tile_count = di + 7;
     c->T.tile_list = c->d_tiles;
+    c->T.tile_max = int(c->scratch_cells) + 1;
     c->T.nscenes = 1;
     c->nbun = nbun;
     c->table_version = c->version;

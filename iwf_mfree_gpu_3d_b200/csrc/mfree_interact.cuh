@@ -917,7 +917,7 @@ __device__ __forceinline__ void produce(const BatchTable &T, BlockSmem &sm, Step
     int slot = 0;
     int2 e = make_int2(0, -1);
     // the first entry is the block's own, the others are claimed
-    const int list_n = *T.tile_count;
+    const int list_n = min(*T.tile_count, T.tile_max);
     if (lane == 0 && int(blockIdx.x) < list_n) e = T.tile_list[blockIdx.x];
     auto claim = [&] {
         if (lane == 0) {

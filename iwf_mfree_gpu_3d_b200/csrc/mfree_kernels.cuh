@@ -93,6 +93,7 @@ struct BatchTable {
     int *tile_next;        // work queue of the pair kernel: next entry of tile_list (reset by kb_clock)
     int *tile_count;       // entries of tile_list (reset by kb_clock)
     int2 *tile_list;       // non-empty pair-kernel tiles of every scene: (tile of the scene, scene * 16 + depth)
+    int tile_max;          // entries it has room for
 };
 
 // Pair-kernel tiles.  A bundle is TX x TY columns of a scene's cell grid
@@ -123,10 +124,20 @@ __host__ __device__ __forceinline__ TileGeo tile_geo(const Params &P, int t, int
 __host__ __device__ __forceinline__ int num_bundles(const Params &P) {
     return ((P.gnx + TX - 1) / TX) * ((P.gny + TY - 1) / TY);
 }
-// an upper bound of a scene's tiles: a tile ends at the depth limit, at the
-// end of its bundle, or because it and its successor hold more than tile_cap
+// Whether a tile of depth > 1 that begins on level z0 is too deep: beyond the
+// depth limit or its bundle's end, with more than tile_cap targets, or with a
+// halo (estimated as four times the bundle's own particles in the halo's
+// levels) beyond TILE_HALO_MAX.  Depth 1 is always taken.
+__host__ __device__ __forceinline__ bool tile_too_deep(const Params &P, int z0, int depth, int targets, int halo) {
+    return depth > P.tile_z || z0 + depth > P.gnz || targets > P.tile_cap || 4 * halo > TILE_HALO_MAX;
+}
+// An upper bound of a scene's tiles, whatever cuts them: each begins on a level
+// of a bundle where no other tile of the bundle begins, and holds a particle.
+// (One counted from the limits alone is not safe: at 70 to 100 particles a
+// level of a bundle the halo cuts every tile to one level, long before tile_cap.)
 inline long long max_tiles(const Params &P) {
-    return (long long)num_bundles(P) * (P.gnz / P.tile_z + 2) + 2ll * P.n_init / P.tile_cap + 2;
+    const long long levels = (long long)num_bundles(P) * P.gnz;
+    return levels < P.n_init ? levels : P.n_init;
 }
 
 // Programmatic dependent launch: a step's kernels are launched while the one

@@ -338,7 +338,7 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
         int k = 0;
         if (lane == 0) k = atomicAdd(T.tile_count, n);
         k = __shfl_sync(0xffffffffu, k, 0);
-        if (lane < n) T.tile_list[k + lane] = mine;
+        if (lane < n && bounds_ok(a.clk, k + lane, T.tile_max)) T.tile_list[k + lane] = mine;
         n = 0;
     };
     for (int z0 = 0; z0 < nz;) {
@@ -355,13 +355,11 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
             z0 = zf;
             continue;  // (the window may have to move)
         }
-        // lane d: would a tile of depth d fit?  Its halo is estimated as four
-        // times the bundle's own particles in the halo's levels.
+        // lane d: would a tile of depth d fit?
         const int d = lane;
         const int in = __shfl_sync(0xffffffffu, F, min(max(min(z0 + d, nz) - base, 0), 31)) - below;
         const int lo = at(max(z0 - 2, 0)), hi = __shfl_sync(0xffffffffu, F, min(max(min(z0 + d + 2, nz) - base, 0), 31));
-        const bool no = d > P.tile_z || z0 + d > nz || in > P.tile_cap || 4 * (hi - lo) > TILE_HALO_MAX;
-        const unsigned bad = __ballot_sync(0xffffffffu, no && d > 1);
+        const unsigned bad = __ballot_sync(0xffffffffu, d > 1 && tile_too_deep(P, z0, d, in, hi - lo));
         const int depth = bad ? __ffs(bad) - 2 : 1;
         if (lane == n) mine = make_int2(bun * nz + z0, s * 16 + depth);
         if (++n == 32) flush();

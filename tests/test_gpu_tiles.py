@@ -78,3 +78,31 @@ def test_results_do_not_depend_on_the_batch_around_a_scene():
         np.testing.assert_array_equal(sims[0].get(n), ref.get(n), err_msg=n)
     ref.close()
     b.close()
+
+
+def test_batch_of_dense_scenes_in_tight_boxes():
+    # h = 1.7 dx and boxes half a spacing around the particles: 84 particles a
+    # level of a bundle, where the halo cuts tiles to one level each -- 1,142
+    # tiles, of which the depth limit and the target count alone would explain
+    # 1,034 at most.  The batch's list must hold them all.
+    def scene(*dims):
+        sc = scenes.orthogonal_cutting(*dims, hdx=1.7)
+        p, m = sc.pos[:, :3], np.float32(0.5e-3)
+        sc.grid_bbmin, sc.grid_bbmax = p.min(0) - m, p.max(0) + m
+        return sc
+
+    dims = ((40, 20, 80), (26, 13, 100))
+    b = api.Batch()
+    sims = [api.Simulation.from_scene(scene(*d)) for d in dims]
+    for s in sims:
+        b.admit(s)
+    b.step(3, record_every=1)
+    b.sync()
+    for s, d in zip(sims, dims):
+        ref = api.Simulation.from_scene(scene(*d))
+        ref.advance(3, record_every=1)
+        for n in ("POS", "VEL", "S", "T", "VEL_T", "ID"):
+            np.testing.assert_array_equal(s.get(n), ref.get(n), err_msg=f"{d}: {n}")
+        assert ref.counts()[0] == ref.counts()[1]
+        ref.close()
+    b.close()

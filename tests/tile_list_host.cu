@@ -1,0 +1,63 @@
+// Host checks of the pair kernel's tile list on its own rules (mfree_kernels.cuh);
+// prints "ok", or what failed.  Needs no GPU.
+#include <cstdio>
+#include <random>
+#include <vector>
+
+#include "mfree_kernels.cuh"
+
+using namespace mfree;
+
+// the tiles of one bundle, cut as the kernel cuts them: empty levels are
+// skipped, and a tile is as deep as the rule allows
+static long long cut(const Params &P, const std::vector<int> &level) {
+    const int nz = P.gnz;
+    std::vector<int> below(nz + 1, 0);
+    for (int z = 0; z < nz; z++) below[z + 1] = below[z] + level[z];
+    auto upto = [&](int z) { return below[z < 0 ? 0 : z > nz ? nz : z]; };
+    long long tiles = 0;
+    for (int z0 = 0; z0 < nz;) {
+        if (level[z0] == 0) {
+            z0++;
+            continue;
+        }
+        int d = 1;
+        while (!tile_too_deep(P, z0, d + 1, upto(z0 + d + 1) - upto(z0), upto(z0 + d + 3) - upto(z0 - 2))) d++;
+        tiles++;
+        z0 += d;
+    }
+    return tiles;
+}
+
+// max_tiles against the tiles of bundles of lo to hi particles a level
+static int check_bound() {
+    std::mt19937 rng(1);
+    const int ranges[][2] = {{0, 1}, {0, 4}, {20, 40}, {60, 110}, {69, 75}, {90, 105}, {100, 500}};
+    for (auto &r : ranges)
+        for (int nz : {1, 2, 9, 33, 100, 257})
+            for (int tile_z : {1, 5, TILE_Z_MAX})
+                for (int cap : {32, 120, 205, 240}) {
+                    Params P{};
+                    P.gnx = 3 * TX - 1, P.gny = 2 * TY, P.gnz = nz;
+                    P.tile_z = tile_z, P.tile_cap = cap;
+                    long long tiles = 0, n = 0;
+                    for (int b = 0; b < num_bundles(P); b++) {
+                        std::vector<int> level(nz);
+                        for (int &l : level) n += l = std::uniform_int_distribution<int>(r[0], r[1])(rng);
+                        tiles += cut(P, level);
+                    }
+                    P.n_init = int(n);
+                    if (tiles > max_tiles(P)) {
+                        printf("%lld tiles, bound %lld: levels of %d to %d, nz %d, tile_z %d, tile_cap %d\n", tiles,
+                               max_tiles(P), r[0], r[1], nz, tile_z, cap);
+                        return 1;
+                    }
+                }
+    return 0;
+}
+
+int main() {
+    if (check_bound()) return 1;
+    printf("ok\n");
+    return 0;
+}
