@@ -124,6 +124,22 @@ __host__ __device__ __forceinline__ TileGeo tile_geo(const Params &P, int t, int
 __host__ __device__ __forceinline__ int num_bundles(const Params &P) {
     return ((P.gnx + TX - 1) / TX) * ((P.gny + TY - 1) / TY);
 }
+// Particles of a bundle on the levels [z0, z), from the cell starts.  (Each
+// column's count is taken before it is added: sixteen cell starts together pass
+// 2^31 from 134M particles on.)
+__host__ __device__ __forceinline__ int bundle_count(const Params &P, const int *__restrict__ first, const TileGeo &G,
+                                                     int z0, int z) {
+    int n = 0;
+#pragma unroll
+    for (int c = 0; c < TX * TY; c++) {
+        const int cx = G.X0 + c / TY, cy = G.Y0 + c % TY;
+        if (cx < P.gnx && cy < P.gny) {
+            const int *col = first + (size_t(cx) * P.gny + cy) * P.gnz;
+            n += col[z] - col[z0];
+        }
+    }
+    return n;
+}
 // Whether a tile of depth > 1 that begins on level z0 is too deep: beyond the
 // depth limit or its bundle's end, with more than tile_cap targets, or with a
 // halo (estimated as four times the bundle's own particles in the halo's

@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(256) k_cell_fixup(StepArgs a) {
 }
 
 // The pair kernel's list of non-empty tiles: one warp per bundle of every
-// scene.  Lane k holds the targets below level base + k of the bundle, so a
-// tile's depth is one ballot over the lanes behind its first level; the
+// scene.  Lane k holds the targets of the bundle from level base to level
+// base + k, so a tile's depth is one ballot over the lanes behind its first level; the
 // bundle's tiles are appended with one atomic per 32 of them.  The order of
 // the list changes which block runs a tile, never a result.
 __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int lane) {
@@ -316,19 +316,13 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
     const int bun = g - T.ibun[s];
     const StepArgs &a = scene_args(T, s);
     const Params &P = a.p;
-    const int nx = P.gnx, ny = P.gny, nz = P.gnz;
+    const int nz = P.gnz;
     const TileGeo G = tile_geo(P, bun * nz, 1);
     const int *__restrict__ first = a.s.first;
     int base = 0, F = 0;
-    auto load = [&](int z) {  // F = targets of the bundle below level z + lane, up to a constant
+    auto load = [&](int z) {  // F = targets of the bundle on the levels z .. z + lane - 1
         base = z;
-        F = 0;
-        const int zz = min(z + lane, nz);
-#pragma unroll
-        for (int c = 0; c < TX * TY; c++) {
-            const int cx = G.X0 + c / TY, cy = G.Y0 + c % TY;
-            if (cx < nx && cy < ny) F += first[(cx * ny + cy) * nz + zz];
-        }
+        F = bundle_count(P, first, G, z, min(z + lane, nz));
     };
     auto at = [&](int z) { return __shfl_sync(0xffffffffu, F, min(z, nz) - base); };
     load(0);

@@ -56,8 +56,30 @@ static int check_bound() {
     return 0;
 }
 
+// bundle_count with cell starts whose sum over a bundle's columns passes 2^31
+static int check_count() {
+    Params P{};
+    P.gnx = 2 * TX + 1, P.gny = TY + 2, P.gnz = 40;
+    std::vector<int> first(size_t(P.gnx) * P.gny * P.gnz + 1);
+    for (long long start : {0ll, 134217700ll, 2147000000ll}) {  // cell 0 begins there; 3 particles a cell
+        for (size_t c = 0; c < first.size(); c++) first[c] = int(start + 3 * (long long)c);
+        for (int b = 0; b < num_bundles(P); b++) {
+            const TileGeo G = tile_geo(P, b * P.gnz, 1);
+            const int cx = P.gnx - G.X0 < TX ? P.gnx - G.X0 : TX, cy = P.gny - G.Y0 < TY ? P.gny - G.Y0 : TY;
+            for (int z0 = 0; z0 <= P.gnz; z0 += 5)
+                for (int z = z0; z <= P.gnz; z++)
+                    if (bundle_count(P, first.data(), G, z0, z) != 3 * cx * cy * (z - z0)) {
+                        printf("bundle %d, levels %d to %d from %lld: %d\n", b, z0, z, start,
+                               bundle_count(P, first.data(), G, z0, z));
+                        return 1;
+                    }
+        }
+    }
+    return 0;
+}
+
 int main() {
-    if (check_bound()) return 1;
+    if (check_bound() || check_count()) return 1;
     printf("ok\n");
     return 0;
 }
