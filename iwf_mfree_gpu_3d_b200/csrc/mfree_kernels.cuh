@@ -124,19 +124,16 @@ __host__ __device__ __forceinline__ TileGeo tile_geo(const Params &P, int t, int
 __host__ __device__ __forceinline__ int num_bundles(const Params &P) {
     return ((P.gnx + TX - 1) / TX) * ((P.gny + TY - 1) / TY);
 }
-// Particles of a bundle on the levels [z0, z), from the cell starts.  (Each
-// column's count is taken before it is added: sixteen cell starts together pass
-// 2^31 from 134M particles on.)
-__host__ __device__ __forceinline__ int bundle_count(const Params &P, const int *__restrict__ first, const TileGeo &G,
-                                                     int z0, int z) {
-    int n = 0;
+// Particles of a bundle below level z, up to a constant: the sum of its columns'
+// cell starts, modulo 2^32 (sixteen of them pass 2^31 from 134M particles on).
+// The difference of two is the number of particles between the levels.
+__host__ __device__ __forceinline__ unsigned bundle_below(const Params &P, const int *__restrict__ first,
+                                                          const TileGeo &G, int z) {
+    unsigned n = 0;
 #pragma unroll
     for (int c = 0; c < TX * TY; c++) {
         const int cx = G.X0 + c / TY, cy = G.Y0 + c % TY;
-        if (cx < P.gnx && cy < P.gny) {
-            const int *col = first + (size_t(cx) * P.gny + cy) * P.gnz;
-            n += col[z] - col[z0];
-        }
+        if (cx < P.gnx && cy < P.gny) n += unsigned(first[(cx * P.gny + cy) * P.gnz + z]);
     }
     return n;
 }

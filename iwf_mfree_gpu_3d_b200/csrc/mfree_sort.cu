@@ -322,7 +322,8 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
     int base = 0, F = 0;
     auto load = [&](int z) {  // F = targets of the bundle on the levels z .. z + lane - 1
         base = z;
-        F = bundle_count(P, first, G, z, min(z + lane, nz));
+        const unsigned n = bundle_below(P, first, G, min(z + lane, nz));
+        F = int(n - __shfl_sync(0xffffffffu, n, 0));
     };
     auto at = [&](int z) { return __shfl_sync(0xffffffffu, F, min(z, nz) - base); };
     load(0);

@@ -56,7 +56,7 @@ static int check_bound() {
     return 0;
 }
 
-// bundle_count with cell starts whose sum over a bundle's columns passes 2^31
+// bundle_below with cell starts whose sum over a bundle's columns passes 2^31
 static int check_count() {
     Params P{};
     P.gnx = 2 * TX + 1, P.gny = TY + 2, P.gnz = 40;
@@ -67,12 +67,13 @@ static int check_count() {
             const TileGeo G = tile_geo(P, b * P.gnz, 1);
             const int cx = P.gnx - G.X0 < TX ? P.gnx - G.X0 : TX, cy = P.gny - G.Y0 < TY ? P.gny - G.Y0 : TY;
             for (int z0 = 0; z0 <= P.gnz; z0 += 5)
-                for (int z = z0; z <= P.gnz; z++)
-                    if (bundle_count(P, first.data(), G, z0, z) != 3 * cx * cy * (z - z0)) {
-                        printf("bundle %d, levels %d to %d from %lld: %d\n", b, z0, z, start,
-                               bundle_count(P, first.data(), G, z0, z));
+                for (int z = z0; z <= P.gnz; z++) {
+                    const int n = int(bundle_below(P, first.data(), G, z) - bundle_below(P, first.data(), G, z0));
+                    if (n != 3 * cx * cy * (z - z0)) {
+                        printf("bundle %d, levels %d to %d from %lld: %d\n", b, z0, z, start, n);
                         return 1;
                     }
+                }
         }
     }
     return 0;
