@@ -318,8 +318,8 @@ int mfree_inject_fault(mfree_ctx *ctx, int kind);
  * bracket every kernel of a step on the context's stream.  Kernel order:
  * clock, hash, scan_reduce, scan_top, scan_down, scatter, cell_fixup,
  * gather_predict, interact, finalize, force_final (MFREE_NUM_KERNELS); the
- * scan is one kernel, counted as scan_down, and scan_reduce, scan_top and
- * cell_fixup are launched no more (0 launches). */
+ * scan is counted as scan_down, preceded by scan_top on grids of more than 16.8M
+ * cells; scan_reduce and cell_fixup are launched no more (0 launches). */
 #define MFREE_NUM_KERNELS 11
 int mfree_set_kernel_timing(mfree_ctx *ctx, int on);
 /* accumulated milliseconds and launch counts per kernel since the last call;

@@ -59,6 +59,7 @@ struct mfree_batch {
     BatchTable T{};
     std::vector<int> run;  // slots in the table, in table order
     int tot_pblk = 0, tot_stile = 0, tot_ibun = 0;
+    bool scan_top = false;  // a scene's scan has more than SCAN_FLAT tiles
     bool dirty = true;
     int table_record_every = -1;
     cudaGraphExec_t graph = nullptr;
@@ -110,6 +111,7 @@ int build_table(mfree_batch *b, int record_every) {
     std::vector<int> pre(3 * size_t(b->cap + 1), 0);
     int *pb = pre.data(), *ps = pb + (b->cap + 1), *pt = ps + (b->cap + 1);
     long long particles = 0, tiles = 0;
+    b->scan_top = false;
     for (int k : b->run) particles += b->slots[k].c->n_init;
     const int cap_targets = default_tile_cap(particles, b->num_sms);
     for (int s = 0; s < n; s++) {
@@ -137,6 +139,7 @@ int build_table(mfree_batch *b, int record_every) {
         ps[s + 1] = ps[s] + scan_tiles(c);
         pt[s + 1] = pt[s] + num_bundles(P);
         tiles += max_tiles(P);
+        if (scan_tiles(c) > SCAN_FLAT) b->scan_top = true;
     }
     b->tot_pblk = pb[n];
     b->tot_stile = ps[n];
@@ -174,6 +177,7 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     };
     run([&] { return launch_after(kb_clock, (n + 127) / 128, 128, 0, s, T, record_mode); });
     run([&] { return launch_after(kb_hash, b->tot_pblk, HASH_BLOCK, 0, s, T); });
+    if (b->scan_top) run([&] { return launch_after(kb_scan_top, n, 1024, 0, s, T); });
     run([&] { return launch_after(kb_scan, b->tot_stile, SCAN_THREADS, 0, s, T); });
     run([&] { return launch_after(kb_scatter, b->tot_pblk + (b->tot_ibun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run([&] { return launch_gather_predict_batch(T, b->prec, b->tot_pblk, s); });

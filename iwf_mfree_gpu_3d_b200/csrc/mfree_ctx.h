@@ -42,7 +42,7 @@ struct TraceRange {
 };
 // the step's kernels in launch order (the ids of mfree_get_kernel_times)
 constexpr const char *KERNEL_TRACE_NAMES[MFREE_NUM_KERNELS] = {
-    "kb_clock", "kb_hash", "", "", "kb_scan", "kb_scatter", "", "kb_gather_predict", "kb_interact", "kb_finalize", "kb_force_final"};
+    "kb_clock", "kb_hash", "", "kb_scan_top", "kb_scan", "kb_scatter", "", "kb_gather_predict", "kb_interact", "kb_finalize", "kb_force_final"};
 
 struct DevTool {
     HostTool host;

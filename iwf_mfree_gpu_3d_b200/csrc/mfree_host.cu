@@ -7,7 +7,7 @@
 // blanking.cpp), leap_frog::step (leap_frog.cu:121-195) and the process globals
 // of mfree_gpu_3d.cpp:41-48.
 //
-// A step is 8 kernels at most on one stream with no host synchronisation (N lives on
+// A step is 9 kernels at most on one stream with no host synchronisation (N lives on
 // the device), so it can also be captured once into a CUDA graph and replayed.
 #include <climits>
 #include <cstdint>
@@ -180,7 +180,7 @@ Params make_params(const mfree_ctx *c) {
 
 static int blank_groups(int n) { return (n + HASH_BLOCK * BLANK_GROUP - 1) / (HASH_BLOCK * BLANK_GROUP); }
 int hash_blocks(const mfree_ctx *c) { return (c->n_init + HASH_BLOCK - 1) / HASH_BLOCK; }
-int scan_tiles(const mfree_ctx *c) { return int((c->num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE); }
+int scan_tiles(const mfree_ctx *c) { return scan_tiles_of(int(c->num_cell)); }
 
 StepArgs make_args(mfree_ctx *c) {
     StepArgs a{};
@@ -380,6 +380,7 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     };
     run(0, [&] { le = launch_after(kb_clock, 1, 32, 0, s, T, record_mode); });
     run(1, [&] { le = launch_after(kb_hash, hb, HASH_BLOCK, 0, s, T); });
+    if (tiles > SCAN_FLAT) run(3, [&] { le = launch_after(kb_scan_top, 1, 1024, 0, s, T); });
     run(4, [&] { le = launch_after(kb_scan, tiles, SCAN_THREADS, 0, s, T); });
     run(5, [&] { le = launch_after(kb_scatter, hb + (c->nbun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run(7, [&] { le = launch_gather_predict_batch(T, P.precision != 0, nb, s); });

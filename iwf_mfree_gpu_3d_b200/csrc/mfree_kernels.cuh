@@ -13,6 +13,13 @@ constexpr int BLANK_GROUP = 128;  // hash blocks per group of blanked counts
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+// Tiles of a scan up to which each of its blocks adds up the tiles before its
+// own; beyond, kb_scan_top scans the tile sums first: the additions grow with
+// the square of the cells, a launch does not.  Scan in us, additions / kb_scan_top
+// (eager event times, some 5 us a kernel are the events'): 8,193 tiles 37 / 42,
+// 16,001 68 / 66, 31,251 151 / 116, 128,001 1,427 / 433.
+constexpr int SCAN_FLAT = 8192;
+__host__ __device__ constexpr int scan_tiles_of(int num_cell) { return (num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE; }
 // blocks of a scene's kb_finalize: one per 256 particles, for many particles
 // eight per SM, each of which looks over more of the contact bitmap (4.1M
 // particles: 16,100 blocks took 54 us to find the few in contact)
@@ -251,6 +258,7 @@ __device__ __forceinline__ void note_blanked(const StepArgs &a, int bid, int nb)
 
 __global__ void kb_clock(BatchTable T, int record_mode);
 __global__ void kb_hash(BatchTable T);
+__global__ void kb_scan_top(BatchTable T);
 __global__ void kb_scan(BatchTable T);
 __global__ void kb_scatter(BatchTable T);
 cudaError_t launch_gather_predict_batch(const BatchTable &T, bool precision, int blocks, cudaStream_t s);

@@ -173,15 +173,47 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &
     return pre + x - v;
 }
 
-// Each block sums the tiles before its own (1,734 at most on the 4.1M-particle
-// scene: seven loads a thread), so the tile sums need no scan of their own.
+// exclusive scan of the tile sums in place, for grids of many tiles
+__device__ __forceinline__ void scan_top_body(const StepArgs &a) {
+    __shared__ int ws[32];
+    constexpr int PER = 8;
+    const int tiles = scan_tiles_of(a.p.num_cell);
+    if (tiles <= SCAN_FLAT) return;
+    int carry = 0;
+    for (int b = 0; b < tiles; b += 1024 * PER) {
+        const int t = b + int(threadIdx.x) * PER;
+        int v[PER], s = 0, total;
+#pragma unroll
+        for (int k = 0; k < PER; k++) s += v[k] = t + k < tiles ? a.s.tile_sum[t + k] : 0;
+        int ex = carry + block_exclusive_scan(s, ws, total);
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            if (t + k < tiles) a.s.tile_sum[t + k] = ex;
+            ex += v[k];
+        }
+        carry += total;
+    }
+}
+// one block per scene
+__global__ void __launch_bounds__(1024) kb_scan_top(BatchTable T) {
+    begin_after();
+    scan_top_body(scene_args(T, blockIdx.x));
+}
+
+// Up to SCAN_FLAT tiles each block sums the tiles before its own (1,734 on the
+// 4.1M-particle scene: seven loads a thread), so the tile sums need no scan.
 __device__ __forceinline__ void scan_body(const StepArgs &a, int bid) {
     __shared__ int ws[32];
     const int nc = a.p.num_cell;
-    int total, before = 0;
-    for (int t = threadIdx.x; t < bid; t += SCAN_THREADS) before += a.s.tile_sum[t];
-    block_exclusive_scan(before, ws, total);
-    const int start = total;
+    int start;
+    if (scan_tiles_of(nc) > SCAN_FLAT) {
+        start = a.s.tile_sum[bid];
+    } else {
+        int before = 0;
+        for (int t = threadIdx.x; t < bid; t += SCAN_THREADS) before += a.s.tile_sum[t];
+        block_exclusive_scan(before, ws, start);
+    }
+    int total;
     const int base = bid * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int s = 0;
@@ -234,7 +266,7 @@ __device__ __forceinline__ void scatter_body(const StepArgs &a, int bid, int *ou
     __shared__ int ws[32];
     const Params &P = a.p;
     {   // the tile sums are done with: zero for the next step
-        const int tiles = (P.num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE, nb = (P.n_init + HASH_BLOCK - 1) / HASH_BLOCK;
+        const int tiles = scan_tiles_of(P.num_cell), nb = (P.n_init + HASH_BLOCK - 1) / HASH_BLOCK;
         for (int t = bid * HASH_BLOCK + threadIdx.x; t < tiles; t += nb * HASH_BLOCK) a.s.tile_sum[t] = 0;
     }
     const int i = bid * HASH_BLOCK + threadIdx.x;

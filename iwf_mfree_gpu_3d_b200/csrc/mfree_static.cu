@@ -30,6 +30,7 @@ namespace {
 constexpr int MAX_N = MFREE_STATIC_MAX_PARTICLES;
 constexpr int MAX_CELLS = MFREE_STATIC_MAX_CELLS;
 constexpr int MAX_TILES = (MAX_CELLS + 1 + SCAN_TILE - 1) / SCAN_TILE + 1;
+static_assert(MAX_TILES <= SCAN_FLAT, "the scan needs no scan of its tile sums");
 constexpr int MAX_GROUPS = (MAX_N + HASH_BLOCK * BLANK_GROUP - 1) / (HASH_BLOCK * BLANK_GROUP);
 constexpr int MAX_HASH_BLOCKS = (MAX_N + HASH_BLOCK - 1) / HASH_BLOCK + 1;
 
