@@ -55,12 +55,14 @@ TOL = {
     # against the FP64 oracle, and so does this path.  These bounds serve
     # where the reference's GPU build is not at hand (grain_vs_ref below).
     "grain_40": dict(POS=0.15, VEL=0.26, S=0.13, EPS_PL=2.4e-2, T=6.8e-2, RHO=4e-3),
-    # the same scene at full size (4.1M particles), 10 steps, where the
-    # reference's GPU build is not at hand: three times 3.5e-2, 1.3e-1, 1.9e-1,
-    # 1.2e-1, 5.0e-2, 2.2e-5, the errors measured with two different pair
-    # kernels (equal to 8 digits: they are the particles of the inside test
-    # above, not the step's rounding)
-    "grain_full_10": dict(POS=0.105, VEL=0.38, S=0.58, EPS_PL=0.35, T=0.152, RHO=6.7e-5),
+    # the same scene at full size (4.1M particles), 10 steps.  Plain FP32
+    # against the FP32 oracle, which takes the same inside decisions
+    # (6.1e-8, 4.2e-7, 2.6e-7, 4.4e-7, 9.2e-7, 1.4e-10)
+    "grain_full_10_fp32": dict(POS=1.9e-7, VEL=1.3e-6, S=8e-7, EPS_PL=1.4e-6, T=2.8e-6, RHO=4.5e-10),
+    # the compensated form against FP64, without the particles within six h of
+    # one that the two pushed differently (1.9e-5, 2.5e-4, 6.7e-5, 1.6e-4,
+    # 1.8e-4, 9.7e-9; with them 3.5e-2, 1.3e-1, 1.9e-1, 1.2e-1, 5.0e-2, 2.2e-5)
+    "grain_full_10_away": dict(POS=6e-5, VEL=7.5e-4, S=2e-4, EPS_PL=5e-4, T=5.5e-4, RHO=3e-8),
     # the CUDA path (plain FP32) against the reference's own GPU step on the
     # grain scenes (measured 40 steps small: 2.3e-6, 4.6e-6, 3.0e-5, 7.5e-7,
     # 1.3e-6, 1.5e-7; 10 steps full size: ~1e-7)
@@ -202,15 +204,24 @@ def hex_block_k(nx: int = 3, ny: int = 2, nz: int = 2, seed: int = 11) -> str:
     return "\n".join(lines) + "\n"
 
 
-def grain_checks(sc_plain, sim_plain, err_vs_fp64: dict, orc_state: dict, steps: int, fallback: str):
+def pushed_differently(sim, orc) -> np.ndarray:
+    """Mask of the particles (by id) whose contact force of the last step is
+    there on one side only, or differs by more than 1 %."""
+    a, b = gpu_state(sim, ["FC"])["FC"], oracle_state(orc, ["FC"])["FC"]
+    na, nb = np.linalg.norm(a, axis=1), np.linalg.norm(b, axis=1)
+    return np.linalg.norm(a - b, axis=1) > 0.01 * np.maximum(na, nb)
+
+
+def grain_checks(sc_plain, sim_plain, err_vs_fp64: dict, orc_state: dict, steps: int, fallback: str = ""):
     """The grain scenes' parity: the CUDA path (plain FP32) against the
     reference's own GPU step, and the error against the FP64 oracle no larger
     than the reference's own (10 % slack) -- or, without the reference's GPU
-    build, the fallback bounds."""
+    build, the fallback bounds (if the scene has any)."""
     from baseline import refgpu
     names = ["POS", "VEL", "S", "EPS_PL", "T", "RHO"]
     if not refgpu.available(refgpu.variant_of(sc_plain)):
-        check(err_vs_fp64, fallback)
+        if fallback:
+            check(err_vs_fp64, fallback)
         return
     st = refgpu.run(sc_plain, 0, steps, state=True)["state"]
     r = {n: by_id(st["ID"], st[n].astype(np.float64)) for n in names + ["BLANKED"]}
