@@ -3,11 +3,12 @@
 A particle in a tool box is served by 2, 8 or 32 lanes, chosen by how many of
 them a block holds and by the triangles of the tools; the closest triangle must
 be the one a serial search keeps.  Scenes with few and with many particles in
-contact, tools on both sides of the triangle limit, both algorithms, particle
-counts that do not fill the bitmap's last word, and tool particles in the
-blanked tail are stepped beside the FP64 oracle: the first contact forces of
+contact, tools on both sides of the triangle limit, both algorithms and particle
+counts that do not fill the bitmap's last word are stepped beside the FP32
+oracle, which takes the same inside decisions: the first contact forces of
 every tool agree to FP32 rounding of the gaps they come from (a last bit of a
-coordinate of 0.04 cm, 4e-9, in a gap of 5e-5 cm: 1e-4 of a force)."""
+coordinate of 0.04 cm, 4e-9, in a gap of 5e-5 cm: 1e-4 of a force).  The same
+kernel moves the tool particles of the blanked tail with their tool."""
 import numpy as np
 import pytest
 
@@ -61,3 +62,30 @@ def test_contact_marks_do_not_outlive_their_step():
     sim.advance(2, record_every=1)
     assert np.abs(sim.get("FC")).max() == 0.0 and np.abs(sim.tool_forces()).max() == 0.0
     sim.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_blanked_tool_particles_move_with_the_tool(precision):
+    sc = scenes.single_grain(22, 18, 9, depth=4.0, radius=6.0, precision=precision, engage=0.8)
+    tool = sc.tool_p == 1
+    x = sc.pos[:, 0]
+    sc.blank_bbmax = sc.blank_bbmax.copy()
+    sc.blank_bbmax[0] = np.median(x[tool])  # half of them are blanked
+    sim = api.Simulation.from_scene(sc)
+    sim.advance(4)
+    ids = sim.get("ID")
+    moved, blanked = np.empty((sc.n, 3)), np.empty(sc.n)
+    moved[ids] = (sim.get64("POS") if precision else sim.get("POS"))[:, :3]
+    blanked[ids] = sim.get("BLANKED")
+    sim.close()
+    tail = tool & (blanked == 1)
+    assert tail.sum() > 300 and (tool & (blanked == 0)).sum() > 300
+    p, v = sc.pos[tail, :3], np.float32(sc.tools[0].vel)
+    if precision:
+        want = p.astype(np.float64) + 4.0 * v.astype(np.float64) * float(np.float32(sc.dt))
+        # high and low parts hold 48 bits; a step moves a particle by 1e-6
+        np.testing.assert_allclose(moved[tail], want, rtol=0.0, atol=1e-12)
+    else:
+        for _ in range(4):  # fmaf(v, dt, p)
+            p = (p.astype(np.float64) + v.astype(np.float64) * float(np.float32(sc.dt))).astype(np.float32)
+        np.testing.assert_array_equal(moved[tail].astype(np.float32), p)
