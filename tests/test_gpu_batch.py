@@ -129,8 +129,8 @@ def test_autotune_leaves_the_scenes_untouched_and_its_tiling_is_used():
     assert b.tiling() == (lpp, depth)
     for s, st in zip(sims, before):
         _assert_same(_state(s), st, "after autotune")
-    # the tuned tiling differs from the default only in rounding; a scene
-    # stepped alone with it from the same state is identical
+    # no result depends on the tiling: a scene stepped alone, first with the
+    # default, then with the tuned one, is identical
     b.step(4, record_every=1)
     ref = api.Simulation.from_scene(_scene(0))
     ref.advance(3, record_every=1)

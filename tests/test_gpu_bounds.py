@@ -1,8 +1,7 @@
 """The bounds-checked debug build (libmfree_checked.so, -DMFREE_BOUNDS_CHECK):
 every index the kernels compute from data -- sort destinations, cell ranges,
-the pair kernel's cell starts, halo staging ranges, target and candidate
-records, the contact triangle ranges --
-is tested against its array and counted when outside, instead of being used.
+the tile list's entries, the pair kernel's cell starts, halo staging ranges, target
+and candidate records, the contact triangle ranges -- is tested against its array and counted when outside, instead of being used.
 Small cases of every kernel variant (and a dense scene whose tiles read their
 records from global memory) run through it in a process of their own
 (the library is loaded once per process): no index may fall outside, and the
@@ -34,7 +33,7 @@ cases = {
     "brookshaw_8k": (scenes.small_scene(), {}),
     "cspm_pse_precision": (scenes.orthogonal_cutting(30, 15, 12, cspm=True, conduction=2), {"precision": 1}),
     "exhaustive_contact": (scenes.orthogonal_cutting(24, 12, 10, algorithm=1), {}),
-    "full_stencil_32_lanes": (scenes.orthogonal_cutting(24, 12, 10), {"full_stencil": 1, "lanes_per_particle": 32}),
+    "full_stencil": (scenes.orthogonal_cutting(24, 12, 10), {"full_stencil": 1}),
 }
 for name, (sc, opt) in cases.items():
     sim = api.Simulation.from_scene(sc, **opt)

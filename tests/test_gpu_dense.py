@@ -1,16 +1,16 @@
 """A dense scene: the pair kernel's paths for tiles that do not fit the staging
 buffer and for targets whose in-support neighbours overflow their queue.
 
-With h = 2.2 dx (the cell edge is h) about ten particles share a cell, so a
-tile's halo (8 x 8 x 10 cells, cut by the block's faces) holds several
-thousand records, more than the staging capacity: every tile of the block
-reads its neighbour records from global memory, with its queues and column
-walks in the idle staging area.  A target has about 350 in-support
-neighbours, more than the 96-entry queue, so the rest are found again by the
-rescan.  Neither happens in the benchmark scenes.  The CUDA path is compared
-with the oracle: one step from a loaded state (every term active) in the
-reference's FP32 semantics, and 5 steps from rest against FP64, for the plain
-and the CSPM + PSE variants (tolerances about 3x the measured errors).
+With h = 2.2 dx (the cell edge is h) about ten particles share a cell.  Tiles
+are cut to one level of 4 x 4 cells then, and the halo of one (8 x 8 x 5 cells,
+cut by the block's faces) still holds more records than the staging area: such
+a tile reads its neighbour records from global memory, with its queues in the
+idle staging area.  A target has about 350 in-support neighbours, more than its
+96-entry queue, so they are found again by the rescan.  Neither happens in the
+benchmark scenes.  The CUDA path is compared with the oracle: one step from a
+loaded state (every term active) in the reference's FP32 semantics, and 5 steps
+from rest against FP64, for the plain and the CSPM + PSE variants (tolerances
+about 3x the measured errors).
 """
 import numpy as np
 import pytest
@@ -28,10 +28,10 @@ def dense_scene(**kw):
 
 
 def test_dense_halo_exceeds_the_staging_capacity():
-    """The premise (host only): tiles of 4 x 4 x 6 cells from the grid origin
-    have halos (8 x 8 x 10 cells) of up to several thousand records, above the
-    staging capacity of 1,788, and a particle's support sphere holds far more
-    than the queue's 96 neighbours."""
+    """The premise (host only): tiles of 4 x 4 x 1 cells from the grid origin
+    have halos (8 x 8 x 5 cells) of up to 2,874 records, more than a block's
+    shared memory holds (232,448 bytes, 96 a record), and a particle's support
+    sphere holds far more than the queue's 96 neighbours."""
     sc = dense_scene()
     p = sc.pos.reshape(sc.n, -1)[:, :3].astype(np.float64)
     lo = np.asarray(sc.grid_bbmin, np.float64)
@@ -39,9 +39,9 @@ def test_dense_halo_exceeds_the_staging_capacity():
     idx = np.floor((p - lo) / h).astype(int)
     cnt = np.zeros(idx.max(0) + 8)
     np.add.at(cnt, tuple(idx.T), 1)
-    halos = [cnt[max(x - 2, 0):x + 6, max(y - 2, 0):y + 6, max(z - 2, 0):z + 8].sum()
-             for x in range(0, cnt.shape[0], 4) for y in range(0, cnt.shape[1], 4) for z in range(0, cnt.shape[2], 6)]
-    assert max(halos) > 2 * 1788, max(halos)
+    halos = [cnt[max(x - 2, 0):x + 6, max(y - 2, 0):y + 6, max(z - 2, 0):z + 3].sum()
+             for x in range(0, cnt.shape[0], 4) for y in range(0, cnt.shape[1], 4) for z in range(cnt.shape[2])]
+    assert max(halos) > 232448 // 96, max(halos)
     assert 4.0 / 3.0 * np.pi * (2 * h / 1.0e-3) ** 3 > 3 * 96  # (2h / dx)^3 lattice sites in the support sphere
 
 
