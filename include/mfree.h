@@ -373,12 +373,12 @@ int mfree_cell_list_static(const float *pos4, int n, const float bbmin[3], float
  * these calls have no counterpart there.  A batch holds independent scenes
  * of any sizes (each an mfree_ctx, configured as for mfree_step) and steps
  * all of them with one launch per kernel: every scene keeps its own state and
- * cell list, and a scene's results are the same alone and in a batch when the
- * pair-loop tiling is the same (and whatever it is).  Scenes are admitted and retired between
- * steps (continuous batching): admission is bounded by a device-memory
- * budget, and a scene may be admitted with a step count after which it stops.
+ * cell list, and a scene's results are the same alone and in a batch, whatever
+ * the pair-loop tiling.  Scenes are admitted and retired between steps
+ * (continuous batching): admission is bounded by a device-memory budget, and a
+ * scene may be admitted with a step count after which it stops.
  * All scenes of a batch share the pair-kernel variant (cspm, conduction,
- * precision options) and the tiling (lanes per particle, tile depth). */
+ * precision options) and the largest tile depth. */
 typedef struct mfree_batch mfree_batch;
 
 /* hbm_budget: device bytes the admitted scenes may hold (0: no limit).
@@ -413,10 +413,10 @@ int mfree_batch_info(mfree_batch *b, int *scenes, int *running, size_t *bytes, s
  * and the largest tile depth (1..8 cells); 0 keeps the current value. */
 int mfree_batch_set_tiling(mfree_batch *b, int lanes_per_particle, int tile_depth);
 int mfree_batch_get_tiling(mfree_batch *b, int *lanes_per_particle, int *tile_depth);
-/* Autotuner: times every largest tile depth (4..8) for
- * trial_steps steps on copies of the batch's running scenes (their own state
- * is untouched) and keeps the fastest.  The cell size stays the reference's
- * (the smoothing length), which the bit-exact cell ids and order require.
+/* Autotuner: times the largest tile depths 4..8 for trial_steps steps on copies
+ * of the batch's running scenes (their own state is untouched) and keeps the
+ * fastest.  The cell size stays the reference's (the smoothing length), which
+ * the bit-exact cell ids and order require.
  * *ms_best: time per step of the chosen tiling (may be NULL). */
 int mfree_batch_autotune(mfree_batch *b, int trial_steps, int *lanes_per_particle, int *tile_depth, double *ms_best);
 /* waits for the batch's queued work; CUDA-event timer on the batch's stream

@@ -16,7 +16,7 @@
 // Scenes join (admit) and leave (retire, or stop at their step count) between
 // steps, bounded by a device-memory budget: continuous batching.  Because
 // every scene's arithmetic is the single-scene step's own code on its own
-// data, a scene's results are the same alone and in a batch for the same
+// data, a scene's results are the same alone and in a batch, whatever the
 // pair-loop tiling.
 #include <algorithm>
 #include <climits>
@@ -47,7 +47,8 @@ struct mfree_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int device = 0, num_sms = 148;
-    int lpp = 8, tile_z = TILE_Z_MAX;
+    int lpp = 8;  // what mfree_batch_get_tiling reports; without effect
+    int tile_z = TILE_Z_MAX;
     bool variant_set = false, cspm = false, prec = false;
     int cond = 0;
     std::vector<Slot> slots;
@@ -247,7 +248,6 @@ int mfree_batch_create(size_t hbm_budget, void *stream, mfree_batch **out) {
         CUDA_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
         b->own_stream = true;
     }
-    b->lpp = default_lpp();
     b->tile_z = default_tile_depth();
     *out = b.release();
     return MFREE_OK;
@@ -451,30 +451,28 @@ int mfree_batch_autotune(mfree_batch *b, int trial_steps, int *lpp_out, int *tz_
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     double best = 1e300;
-    int blpp = b->lpp, btz = b->tile_z;
-    const int lpp = 8;  // the pair kernel has one mapping of lanes to particles
-        for (int tz = 4; tz <= TILE_Z_MAX && !st; tz++) {
-            if ((st = mfree_batch_set_tiling(tb, lpp, tz))) break;
-            if ((st = mfree_batch_step(tb, 1, 0, 1))) break;  // capture + warm-up
-            cudaEventRecord(e0, b->stream);
-            if ((st = mfree_batch_step(tb, trial_steps, 0, 1))) break;
-            cudaEventRecord(e1, b->stream);
-            cudaEventSynchronize(e1);
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (ms < best) {
-                best = ms;
-                blpp = lpp;
-                btz = tz;
-            }
+    int btz = b->tile_z;
+    for (int tz = 4; tz <= TILE_Z_MAX; tz++) {
+        if ((st = mfree_batch_set_tiling(tb, 0, tz))) break;
+        if ((st = mfree_batch_step(tb, 1, 0, 1))) break;  // capture + warm-up
+        cudaEventRecord(e0, b->stream);
+        if ((st = mfree_batch_step(tb, trial_steps, 0, 1))) break;
+        cudaEventRecord(e1, b->stream);
+        cudaEventSynchronize(e1);
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, e0, e1);
+        if (ms < best) {
+            best = ms;
+            btz = tz;
         }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (st) return st;
-    b->lpp = blpp;
+    b->lpp = 8;
     b->tile_z = btz;
     b->dirty = true;
-    if (lpp_out) *lpp_out = blpp;
+    if (lpp_out) *lpp_out = b->lpp;
     if (tz_out) *tz_out = btz;
     if (ms_best) *ms_best = best / trial_steps;
     return MFREE_OK;

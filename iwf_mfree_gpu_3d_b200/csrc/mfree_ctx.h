@@ -133,7 +133,6 @@ struct mfree_ctx {
 namespace mfree {
 namespace host {
 
-int default_lpp();
 int default_tile_depth();
 int default_tile_cap(long long n, int num_sms);
 int hash_blocks(const mfree_ctx *c);

@@ -195,18 +195,6 @@ struct alignas(16) StepArgs {
 
 __device__ __forceinline__ bool nan_or_inf(float v) { return isnan(v) || isinf(v); }
 
-// r^2 in the unfused order ((dx*dx + dy*dy) + dz*dz): the neighbour-count
-// definition shared with the oracle
-__device__ __forceinline__ float dist2_rn(float dx, float dy, float dz) {
-    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-}
-// 1e-8 <= r^2 < 4 h^2 (kernels.cuh:41); the reference compares the float r^2
-// with the double literal 1e-8, i.e. r^2 > 9.99999994e-9f (largest float below 1e-8)
-__device__ __forceinline__ bool in_support(float r2, float h) {
-    float four_h2 = __fmul_rn(__fmul_rn(4.0f, h), h);
-    return !(r2 >= four_h2) && (r2 > 9.99999994e-9f);
-}
-
 // ------------------------------------------------------ eigen solver ----
 // Eberly's robust symmetric 3x3 eigensolver with the branch choices of
 // src/eigen_solver.cu:19-302 (eigenvalues ascending, right-handed vectors).

@@ -94,7 +94,6 @@ void invalidate_graphs(mfree_ctx *c) {
     c->graph_record_every = -1;
 }
 
-int default_lpp() { return 8; }
 int default_tile_depth() { return TILE_Z_MAX; }
 // Targets a tile should hold.  A block serves 240 at once (mfree_interact.cuh),
 // a tile comes out about 70 % full (levels of a bundle are not divided, bundles

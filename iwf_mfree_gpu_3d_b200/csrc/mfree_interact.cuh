@@ -785,8 +785,9 @@ __device__ __forceinline__ int process_target(const StepArgs &a, const TileTab &
     const int qstep = sl == 0 ? 1 : -1;
     int qn = 0;
     float pse = 0.f;
-    // the in-support test of the reference's neighbour count: the unfused sum
-    // of squares, 1e-8 <= r^2 < 4 h^2
+    // the in-support test of the reference's neighbour count (kernels.cuh:41): the
+    // unfused sum of squares, 1e-8 <= r^2 < 4 h^2, the lower bound a double
+    // there: r^2 > 9.99999994e-9f, the largest float below it
     auto dist2 = [&](const float4 Pj) {
         const float2 d = add2(lo2(Pj), I.nxy);
         const float dz = Pj.z + I.nz;

@@ -21,11 +21,11 @@ constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr int SCAN_FLAT = 8192;
 __host__ __device__ constexpr int scan_tiles_of(int num_cell) { return (num_cell + 1 + SCAN_TILE - 1) / SCAN_TILE; }
 // blocks of a scene's kb_finalize: one per 256 particles, for many particles
-// eight per SM, each of which looks over more of the contact bitmap (4.1M
+// eight per SM (of 148), each of which looks over more of the contact bitmap (4.1M
 // particles: 16,100 blocks took 54 us to find the few in contact)
-constexpr int FIN_BLOCK = 256;
+constexpr int FIN_BLOCK = 256, FIN_BLOCKS_MAX = 8 * 148;
 __host__ __device__ constexpr int finalize_blocks(int n) {
-    return (n + FIN_BLOCK - 1) / FIN_BLOCK < 1184 ? (n + FIN_BLOCK - 1) / FIN_BLOCK : 1184;
+    return (n + FIN_BLOCK - 1) / FIN_BLOCK < FIN_BLOCKS_MAX ? (n + FIN_BLOCK - 1) / FIN_BLOCK : FIN_BLOCKS_MAX;
 }
 constexpr int NRES = 20;           // reduced accumulators per particle
 
