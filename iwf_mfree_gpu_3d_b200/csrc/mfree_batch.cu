@@ -178,8 +178,8 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     };
     run([&] { return launch_after(kb_clock, (n + 127) / 128, 128, 0, s, T, record_mode); });
     run([&] { return launch_after(kb_hash, b->tot_pblk, HASH_BLOCK, 0, s, T); });
-    if (b->scan_top) run([&] { return launch_after(kb_scan_top, n, 1024, 0, s, T); });
-    run([&] { return launch_after(kb_scan, b->tot_stile, SCAN_THREADS, 0, s, T); });
+    if (b->scan_top) run([&] { return launch_scan_top_batch(T, s); });
+    run([&] { return launch_scan_batch(T, b->scan_top, b->tot_stile, s); });
     run([&] { return launch_after(kb_scatter, b->tot_pblk + (b->tot_ibun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run([&] { return launch_gather_predict_batch(T, b->prec, b->tot_pblk, s); });
     run([&] { return launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s); });

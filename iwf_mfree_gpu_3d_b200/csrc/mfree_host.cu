@@ -379,8 +379,9 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     };
     run(0, [&] { le = launch_after(kb_clock, 1, 32, 0, s, T, record_mode); });
     run(1, [&] { le = launch_after(kb_hash, hb, HASH_BLOCK, 0, s, T); });
-    if (tiles > SCAN_FLAT) run(3, [&] { le = launch_after(kb_scan_top, 1, 1024, 0, s, T); });
-    run(4, [&] { le = launch_after(kb_scan, tiles, SCAN_THREADS, 0, s, T); });
+    const bool scan_top = tiles > SCAN_FLAT;
+    if (scan_top) run(3, [&] { le = launch_scan_top_batch(T, s); });
+    run(4, [&] { le = launch_scan_batch(T, scan_top, tiles, s); });
     run(5, [&] { le = launch_after(kb_scatter, hb + (c->nbun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run(7, [&] { le = launch_gather_predict_batch(T, P.precision != 0, nb, s); });
     run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });

@@ -258,8 +258,9 @@ __device__ __forceinline__ void note_blanked(const StepArgs &a, int bid, int nb)
 
 __global__ void kb_clock(BatchTable T, int record_mode);
 __global__ void kb_hash(BatchTable T);
-__global__ void kb_scan_top(BatchTable T);
-__global__ void kb_scan(BatchTable T);
+// top: a scene has more than SCAN_FLAT tiles (launch_scan_top_batch comes first then)
+cudaError_t launch_scan_top_batch(const BatchTable &T, cudaStream_t s);
+cudaError_t launch_scan_batch(const BatchTable &T, bool top, int blocks, cudaStream_t s);
 __global__ void kb_scatter(BatchTable T);
 cudaError_t launch_gather_predict_batch(const BatchTable &T, bool precision, int blocks, cudaStream_t s);
 __global__ void kb_finalize(BatchTable T);

@@ -202,18 +202,18 @@ __global__ void __launch_bounds__(1024) kb_scan_top(BatchTable T) {
 
 // Up to SCAN_FLAT tiles each block sums the tiles before its own (1,734 on the
 // 4.1M-particle scene: seven loads a thread), so the tile sums need no scan.
-__device__ __forceinline__ void scan_body(const StepArgs &a, int bid) {
+// TOP: kb_scan_top has run and scanned those of scenes of more tiles.
+template <bool TOP> __device__ __forceinline__ void scan_body(const StepArgs &a, int bid) {
     __shared__ int ws[32];
     const int nc = a.p.num_cell;
-    int start;
-    if (scan_tiles_of(nc) > SCAN_FLAT) {
-        start = a.s.tile_sum[bid];
-    } else {
-        int before = 0;
+    int total, before = 0;
+    const bool scanned = TOP && scan_tiles_of(nc) > SCAN_FLAT;
+    if (!scanned)
         for (int t = threadIdx.x; t < bid; t += SCAN_THREADS) before += a.s.tile_sum[t];
-        block_exclusive_scan(before, ws, start);
-    }
-    int total;
+    else if (threadIdx.x == 0)
+        before = a.s.tile_sum[bid];
+    block_exclusive_scan(before, ws, total);
+    const int start = total;
     const int base = bid * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
     int s = 0;
@@ -253,11 +253,11 @@ __device__ __forceinline__ void scan_body(const StepArgs &a, int bid) {
 }
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan(StepArgs a) {
     begin_after();
-    scan_body(a, blockIdx.x);
+    scan_body<false>(a, blockIdx.x);
 }
-__global__ void __launch_bounds__(SCAN_THREADS) kb_scan(BatchTable T) {
+template <bool TOP> __global__ void __launch_bounds__(SCAN_THREADS) kb_scan(BatchTable T) {
     begin_after();
-    run_batched(T, T.stile, [](const StepArgs &a, int b) { scan_body(a, b); });
+    run_batched(T, T.stile, [](const StepArgs &a, int b) { scan_body<TOP>(a, b); });
 }
 
 // ---------------------------------------------------------- the scatter --
@@ -522,6 +522,12 @@ cudaError_t launch_init_state(int n, const float4 *pos, const float4 *vel, const
     return cudaGetLastError();
 }
 
+cudaError_t launch_scan_top_batch(const BatchTable &T, cudaStream_t s) {
+    return launch_after(kb_scan_top, T.nscenes, 1024, 0, s, T);
+}
+cudaError_t launch_scan_batch(const BatchTable &T, bool top, int blocks, cudaStream_t s) {
+    return launch_after(top ? kb_scan<true> : kb_scan<false>, blocks, SCAN_THREADS, 0, s, T);
+}
 cudaError_t launch_gather_predict_batch(const BatchTable &T, bool precision, int blocks, cudaStream_t s) {
     return launch_after(precision ? kb_gather_predict<true> : kb_gather_predict<false>, blocks, 256, 0, s, T);
 }
