@@ -57,10 +57,10 @@ struct mfree_batch {
     int cap = 0;
     int2 *d_tiles = nullptr;  // the pair kernel's tile list over every scene
     long long tiles_cap = 0;
+    bool scan_top = false;  // a scene's scan has more than SCAN_FLAT tiles
     BatchTable T{};
     std::vector<int> run;  // slots in the table, in table order
-    int tot_pblk = 0, tot_stile = 0, tot_ibun = 0;
-    bool scan_top = false;  // a scene's scan has more than SCAN_FLAT tiles
+    int tot_pblk = 0, tot_stile = 0, tot_irun = 0;
     bool dirty = true;
     int table_record_every = -1;
     cudaGraphExec_t graph = nullptr;
@@ -105,7 +105,7 @@ int build_table(mfree_batch *b, int record_every) {
     b->T.args = dargs;
     b->T.pblk = dint;
     b->T.stile = dint + (b->cap + 1);
-    b->T.ibun = dint + 2 * (b->cap + 1);
+    b->T.irun = dint + 2 * (b->cap + 1);
     b->T.tile_next = dint + 3 * (b->cap + 1);
     b->T.tile_count = dint + 3 * (b->cap + 1) + 1;
     std::vector<StepArgs> args(2 * size_t(n));
@@ -138,13 +138,13 @@ int build_table(mfree_batch *b, int record_every) {
         const Params &P = args[2 * s].p;
         pb[s + 1] = pb[s] + hash_blocks(c);
         ps[s + 1] = ps[s] + scan_tiles(c);
-        pt[s + 1] = pt[s] + num_bundles(P);
+        pt[s + 1] = pt[s] + num_bundles(P) * bundle_runs(P);
         tiles += max_tiles(P);
         if (scan_tiles(c) > SCAN_FLAT) b->scan_top = true;
     }
     b->tot_pblk = pb[n];
     b->tot_stile = ps[n];
-    b->tot_ibun = pt[n];
+    b->tot_irun = pt[n];
     if (tiles > b->tiles_cap) {  // the tile list of all scenes
         CUDA_TRY(cudaStreamSynchronize(b->stream));  // the old list may still be read
         const long long cap = std::max(tiles, 2 * b->tiles_cap);
@@ -180,7 +180,7 @@ int enqueue_batch_step(mfree_batch *b, int record_mode) {
     run([&] { return launch_after(kb_hash, b->tot_pblk, HASH_BLOCK, 0, s, T); });
     if (b->scan_top) run([&] { return launch_scan_top_batch(T, s); });
     run([&] { return launch_scan_batch(T, b->scan_top, b->tot_stile, s); });
-    run([&] { return launch_after(kb_scatter, b->tot_pblk + (b->tot_ibun + 7) / 8, HASH_BLOCK, 0, s, T); });
+    run([&] { return launch_after(kb_scatter, b->tot_pblk + (b->tot_irun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run([&] { return launch_gather_predict_batch(T, b->prec, b->tot_pblk, s); });
     run([&] { return launch_interact_batch(T, b->cspm, b->cond, b->prec, b->num_sms, s); });
     run([&] { return launch_after(kb_finalize, b->tot_pblk, FIN_BLOCK, 0, s, T); });

@@ -115,7 +115,7 @@ struct mfree_ctx {
     // one-scene table of the batched kernels (ensure_table)
     unsigned char *d_table = nullptr;
     int2 *d_tiles = nullptr;  // the pair kernel's list of non-empty tiles (grid-sized scratch)
-    int nbun = 0;             // bundles of tiles of the grid
+    int nrun = 0;             // runs of tiles of the grid
     mfree::BatchTable T{};
     unsigned long long table_version = ~0ull;
     int table_record_every = -1;

@@ -329,8 +329,8 @@ int ensure_table(mfree_ctx *c, int record_every) {
     }
     c->cur = keep;
     const Params &P = args[0].p;
-    const int nbun = num_bundles(P);
-    const int pre[8] = {0, hash_blocks(c), 0, scan_tiles(c), 0, nbun, 0, 0};
+    const int nrun = num_bundles(P) * bundle_runs(P);
+    const int pre[8] = {0, hash_blocks(c), 0, scan_tiles(c), 0, nrun, 0, 0};
     StepArgs *da = (StepArgs *)c->d_table;
     int *di = (int *)(da + 2);
     // pageable sources: the call returns once the bytes are staged
@@ -339,13 +339,13 @@ int ensure_table(mfree_ctx *c, int record_every) {
     c->T.args = da;
     c->T.pblk = di;
     c->T.stile = di + 2;
-    c->T.ibun = di + 4;
+    c->T.irun = di + 4;
     c->T.tile_next = di + 6;
     c->T.tile_count = di + 7;
     c->T.tile_list = c->d_tiles;
     c->T.tile_max = int(c->scratch_cells) + 1;
     c->T.nscenes = 1;
-    c->nbun = nbun;
+    c->nrun = nrun;
     c->table_version = c->version;
     c->table_record_every = record_every;
     return MFREE_OK;
@@ -382,7 +382,7 @@ int enqueue_step(mfree_ctx *c, int record_mode, int record_every, bool timed = f
     const bool scan_top = tiles > SCAN_FLAT;
     if (scan_top) run(3, [&] { le = launch_scan_top_batch(T, s); });
     run(4, [&] { le = launch_scan_batch(T, scan_top, tiles, s); });
-    run(5, [&] { le = launch_after(kb_scatter, hb + (c->nbun + 7) / 8, HASH_BLOCK, 0, s, T); });
+    run(5, [&] { le = launch_after(kb_scatter, hb + (c->nrun + 7) / 8, HASH_BLOCK, 0, s, T); });
     run(7, [&] { le = launch_gather_predict_batch(T, P.precision != 0, nb, s); });
     run(8, [&] { le = launch_interact_batch(T, P.cspm != 0, P.conduction, P.precision != 0, c->num_sms, s); });
     run(9, [&] { le = launch_after(kb_finalize, finalize_blocks(c->n_init), FIN_BLOCK, 0, s, T); });

@@ -95,7 +95,7 @@ struct BatchTable {
     const StepArgs *args;  // [2 s + parity]
     const int *pblk;       // particle blocks of 256 threads (hash, scatter, gather, finalize)
     const int *stile;      // scan tiles of SCAN_TILE cells
-    const int *ibun;       // bundles of pair-kernel tiles
+    const int *irun;       // runs of pair-kernel tiles
     int nscenes;
     int *tile_next;        // work queue of the pair kernel: next entry of tile_list (reset by kb_clock)
     int *tile_count;       // entries of tile_list (reset by kb_clock)
@@ -110,7 +110,10 @@ struct BatchTable {
 // or thin regions too (tiles of a fixed depth held 156 targets of the 211 of a
 // full one on the 1M-particle block).
 // A tile is named by bundle * gnz + its first level, and its depth.
-constexpr int TX = 4, TY = 4;
+// The cutting is one chain of some 0.4 us a tile, so a bundle is cut in runs of
+// TILE_RUN levels, each by a warp of its own (4 x 4 x 2000 particles, a step:
+// 244 us as one run, 106 us as thirteen).
+constexpr int TX = 4, TY = 4, TILE_RUN = 128;
 constexpr int TILE_HALO_MAX = 1640;  // records the halo of a tile should hold at most (estimated from its bundle)
 struct TileGeo {
     int X0, Y0, Z0, zl, nzr, depth;
@@ -131,25 +134,27 @@ __host__ __device__ __forceinline__ TileGeo tile_geo(const Params &P, int t, int
 __host__ __device__ __forceinline__ int num_bundles(const Params &P) {
     return ((P.gnx + TX - 1) / TX) * ((P.gny + TY - 1) / TY);
 }
+__host__ __device__ __forceinline__ int bundle_runs(const Params &P) { return (P.gnz + TILE_RUN - 1) / TILE_RUN; }
 // Particles of a bundle below level z, up to a constant: the sum of its columns'
 // cell starts, modulo 2^32 (sixteen of them pass 2^31 from 134M particles on).
 // The difference of two is the number of particles between the levels.
-__host__ __device__ __forceinline__ unsigned bundle_below(const Params &P, const int *__restrict__ first,
+__host__ __device__ __forceinline__ unsigned bundle_below(int nx, int ny, int nz, const int *__restrict__ first,
                                                           const TileGeo &G, int z) {
     unsigned n = 0;
 #pragma unroll
     for (int c = 0; c < TX * TY; c++) {
         const int cx = G.X0 + c / TY, cy = G.Y0 + c % TY;
-        if (cx < P.gnx && cy < P.gny) n += unsigned(first[(cx * P.gny + cy) * P.gnz + z]);
+        if (cx < nx && cy < ny) n += unsigned(first[(cx * ny + cy) * nz + z]);
     }
     return n;
 }
 // Whether a tile of depth > 1 that begins on level z0 is too deep: beyond the
-// depth limit or its bundle's end, with more than tile_cap targets, or with a
+// depth limit or the end of its run, with more than tile_cap targets, or with a
 // halo (estimated as four times the bundle's own particles in the halo's
 // levels) beyond TILE_HALO_MAX.  Depth 1 is always taken.
-__host__ __device__ __forceinline__ bool tile_too_deep(const Params &P, int z0, int depth, int targets, int halo) {
-    return depth > P.tile_z || z0 + depth > P.gnz || targets > P.tile_cap || 4 * halo > TILE_HALO_MAX;
+__host__ __device__ __forceinline__ bool tile_too_deep(const Params &P, int z0, int z_end, int depth,
+                                                       int targets, int halo) {
+    return depth > P.tile_z || z0 + depth > z_end || targets > P.tile_cap || 4 * halo > TILE_HALO_MAX;
 }
 // An upper bound of a scene's tiles, whatever cuts them: each begins on a level
 // of a bundle where no other tile of the bundle begins, and holds a particle.

@@ -337,28 +337,30 @@ __global__ void __launch_bounds__(256) k_cell_fixup(StepArgs a) {
     cell_fixup_body(a, blockIdx.x);
 }
 
-// The pair kernel's list of non-empty tiles: one warp per bundle of every
-// scene.  Lane k holds the targets of the bundle from level base to level
-// base + k, so a tile's depth is one ballot over the lanes behind its first level; the
-// bundle's tiles are appended with one atomic per 32 of them.  The order of
-// the list changes which block runs a tile, never a result.
+// The pair kernel's list of non-empty tiles: one warp per run of a bundle of
+// every scene.  Lane k holds bundle_below of level base + k, so a tile's depth
+// is one ballot over the lanes behind its first level; the run's tiles are
+// appended with one atomic per 32 of them.  The order of the list changes which
+// block runs a tile, never a result.
 __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int lane) {
-    if (g >= T.ibun[T.nscenes]) return;
-    const int s = find_scene(T.ibun, T.nscenes, g);
-    const int bun = g - T.ibun[s];
+    if (g >= T.irun[T.nscenes]) return;
+    const int s = find_scene(T.irun, T.nscenes, g);
     const StepArgs &a = scene_args(T, s);
     const Params &P = a.p;
-    const int nz = P.gnz;
+    const int nx = P.gnx, ny = P.gny, nz = P.gnz, nb = num_bundles(P);
+    int bun = g - T.irun[s], z_begin = 0;  // the bundles' first runs come first, then their second ones
+    for (; bun >= nb; bun -= nb) z_begin += TILE_RUN;
+    const int z_end = min(z_begin + TILE_RUN, nz);
     const TileGeo G = tile_geo(P, bun * nz, 1);
     const int *__restrict__ first = a.s.first;
-    int base = 0, F = 0;
-    auto load = [&](int z) {  // F = targets of the bundle on the levels z .. z + lane - 1
+    int base = 0;
+    unsigned F = 0;
+    auto load = [&](int z) {
         base = z;
-        const unsigned n = bundle_below(P, first, G, min(z + lane, nz));
-        F = int(n - __shfl_sync(0xffffffffu, n, 0));
+        F = bundle_below(nx, ny, nz, first, G, min(z + lane, nz));
     };
     auto at = [&](int z) { return __shfl_sync(0xffffffffu, F, min(z, nz) - base); };
-    load(0);
+    load(max(z_begin - 2, 0));
     int2 mine = make_int2(0, 0);
     int n = 0;
     auto flush = [&] {
@@ -368,11 +370,11 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
         if (lane < n && bounds_ok(a.clk, k + lane, T.tile_max)) T.tile_list[k + lane] = mine;
         n = 0;
     };
-    for (int z0 = 0; z0 < nz;) {
+    for (int z0 = z_begin; z0 < z_end;) {
         if (min(z0 + TILE_Z_MAX + 2, nz) > base + 31) load(max(z0 - 2, 0));
         // the first level with a target (a level past the window: look again there)
-        const int below = at(z0);
-        const unsigned some = __ballot_sync(0xffffffffu, base + lane > z0 && base + lane <= nz && F > below);
+        const unsigned below = at(z0);
+        const unsigned some = __ballot_sync(0xffffffffu, base + lane > z0 && base + lane <= nz && int(F - below) > 0);
         if (some == 0) {
             z0 = base + 31;
             continue;
@@ -384,9 +386,9 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
         }
         // lane d: would a tile of depth d fit?
         const int d = lane;
-        const int in = __shfl_sync(0xffffffffu, F, min(max(min(z0 + d, nz) - base, 0), 31)) - below;
-        const int lo = at(max(z0 - 2, 0)), hi = __shfl_sync(0xffffffffu, F, min(max(min(z0 + d + 2, nz) - base, 0), 31));
-        const unsigned bad = __ballot_sync(0xffffffffu, d > 1 && tile_too_deep(P, z0, d, in, hi - lo));
+        const int in = int(__shfl_sync(0xffffffffu, F, min(max(min(z0 + d, nz) - base, 0), 31)) - below);
+        const int halo = int(__shfl_sync(0xffffffffu, F, min(max(min(z0 + d + 2, nz) - base, 0), 31)) - at(max(z0 - 2, 0)));
+        const unsigned bad = __ballot_sync(0xffffffffu, d > 1 && tile_too_deep(P, z0, z_end, d, in, halo));
         const int depth = bad ? __ffs(bad) - 2 : 1;
         if (lane == n) mine = make_int2(bun * nz + z0, s * 16 + depth);
         if (++n == 32) flush();
@@ -399,7 +401,7 @@ __device__ __forceinline__ void tile_list_body(const BatchTable &T, int g, int l
 // has run), the others scatter
 __global__ void __launch_bounds__(HASH_BLOCK) kb_scatter(BatchTable T) {
     begin_after();
-    const int tb = (T.ibun[T.nscenes] + 7) / 8, b = int(blockIdx.x) - tb;
+    const int tb = (T.irun[T.nscenes] + 7) / 8, b = int(blockIdx.x) - tb;
     if (b < 0) {
         tile_list_body(T, int(blockIdx.x) * 8 + int(threadIdx.x >> 5), int(threadIdx.x & 31));
         return;

@@ -10,9 +10,10 @@ sized by the particles of all its scenes.
 import numpy as np
 import pytest
 
+import oracle
 from iwf_mfree_gpu_3d_b200 import api, scenes
 
-from helpers import loaded
+from helpers import compare, gpu_state, loaded, oracle_state
 
 pytestmark = pytest.mark.gpu
 
@@ -61,6 +62,42 @@ def test_results_do_not_depend_on_the_tiles(case):
         assert ref["NUM_NBH"].max() > 96  # beyond a queue's capacity
     for depth in (1, 2, 5, 7):
         _same(ref, _state(CASES[case](), 3, tile_depth=depth), f"{case}, depth {depth}")
+
+
+def test_tall_grids_against_the_oracle():
+    # bundles of more levels than one warp cuts: every level must be in a tile
+    for dims in ((4, 5, 400), (9, 3, 170)):
+        sc = loaded(scenes.orthogonal_cutting(*dims, cspm=True, conduction=1))
+        sim = api.Simulation.from_scene(sc, diagnostics=1)
+        assert sim.grid()[0][2] > 128
+        orc = oracle.Oracle(sc, prec=32)
+        sim.step()
+        orc.step()
+        assert sim.get("NUM_NBH").min() > 0
+        err = compare(gpu_state(sim), oracle_state(orc), sc)
+        sim.close()
+        assert err["blank_mismatch"] == 0
+        for k in ("POS", "VEL", "RHO", "VEL_T", "POS_T", "RHO_T", "S_T"):
+            assert err[k] < 2e-5, (dims, k, err)
+
+
+def test_tall_and_long_blocks_take_about_as_long():
+    # the same block lying and standing (it stood 2.2 times as long while one
+    # warp cut all the tiles above one another)
+    def ms(*dims):
+        sim = api.Simulation.from_scene(scenes.orthogonal_cutting(*dims))
+        sim.advance(3)
+        sim.sync()
+        t = []
+        for _ in range(3):
+            sim.timer_start()
+            sim.advance(20)
+            t.append(sim.timer_stop() / 20)
+        sim.close()
+        return min(t)
+
+    tall, long = ms(4, 4, 2000), ms(2000, 4, 4)
+    assert tall < 1.7 * long, (tall, long)
 
 
 def test_results_do_not_depend_on_the_batch_around_a_scene():

@@ -1,5 +1,6 @@
 // Host checks of the pair kernel's tile list on its own rules (mfree_kernels.cuh);
 // prints "ok", or what failed.  Needs no GPU.
+#include <algorithm>
 #include <cstdio>
 #include <random>
 #include <vector>
@@ -8,8 +9,8 @@
 
 using namespace mfree;
 
-// the tiles of one bundle, cut as the kernel cuts them: empty levels are
-// skipped, and a tile is as deep as the rule allows
+// the tiles of one bundle, cut as the kernel cuts them: in runs, where empty
+// levels are skipped, and a tile is as deep as the rule allows
 static long long cut(const Params &P, const std::vector<int> &level) {
     const int nz = P.gnz;
     std::vector<int> below(nz + 1, 0);
@@ -22,7 +23,8 @@ static long long cut(const Params &P, const std::vector<int> &level) {
             continue;
         }
         int d = 1;
-        while (!tile_too_deep(P, z0, d + 1, upto(z0 + d + 1) - upto(z0), upto(z0 + d + 3) - upto(z0 - 2))) d++;
+        const int z_end = std::min((z0 / TILE_RUN + 1) * TILE_RUN, nz);
+        while (!tile_too_deep(P, z0, z_end, d + 1, upto(z0 + d + 1) - upto(z0), upto(z0 + d + 3) - upto(z0 - 2))) d++;
         tiles++;
         z0 += d;
     }
@@ -68,7 +70,7 @@ static int check_count() {
             const int cx = P.gnx - G.X0 < TX ? P.gnx - G.X0 : TX, cy = P.gny - G.Y0 < TY ? P.gny - G.Y0 : TY;
             for (int z0 = 0; z0 <= P.gnz; z0 += 5)
                 for (int z = z0; z <= P.gnz; z++) {
-                    const int n = int(bundle_below(P, first.data(), G, z) - bundle_below(P, first.data(), G, z0));
+                    const int n = int(bundle_below(P.gnx, P.gny, P.gnz, first.data(), G, z) - bundle_below(P.gnx, P.gny, P.gnz, first.data(), G, z0));
                     if (n != 3 * cx * cy * (z - z0)) {
                         printf("bundle %d, levels %d to %d from %lld: %d\n", b, z0, z, start, n);
                         return 1;
