@@ -410,8 +410,12 @@ __device__ __forceinline__ void finalize_body(const StepArgs &a, int bid) {
         // Few triangles: as wide a group as lets the block take all its
         // particles at once (8,000 particles and a wedge, a step's contact:
         // 2 lanes 15 us, 32 lanes 32 us).  Many: narrow groups read unrelated
-        // triangles and wait for the longest of sixteen searches (five grains:
-        // 32 lanes 137 us, 2 lanes 342 us, before the words were dealt out).
+        // triangles and wait for the longest of sixteen searches.  num_tris counts
+        // a hashed mesh's triangles once for every cell that holds them.  us by
+        // count / 32 lanes, on five small grains, one deep grain (some 500
+        // particles in contact) and a large one (some 2,000): 291 triangles
+        // 53/30, 54/74, 106/106; 1,345 66/33, 65/81, 128/124; 5,720 87/48,
+        // 110/81, 154/124; 320 exhaustive 41/31, 83/71.
         bool many = false;
         for (int k = 0; k < P.num_tools; k++) many |= a.tools[k].num_tris > 512;
         if (many || n <= FIN_BLOCK / 32) take(Group<32>(lane));
