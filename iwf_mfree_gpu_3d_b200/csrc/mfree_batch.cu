@@ -146,12 +146,15 @@ int build_table(mfree_batch *b, int record_every) {
     b->tot_stile = ps[n];
     b->tot_irun = pt[n];
     if (tiles > b->tiles_cap) {  // the tile list of all scenes
-        CUDA_TRY(cudaStreamSynchronize(b->stream));  // the old list may still be read
         const long long cap = std::max(tiles, 2 * b->tiles_cap);
-        if (b->d_tiles) cudaFree(b->d_tiles);
+        cudaMemPool_t pool = context_pool(b->device);
+        if (!pool) return fail(MFREE_ERR_CUDA, "cudaMemPoolCreate failed");
+        if (b->d_tiles) cudaFreeAsync(b->d_tiles, b->stream);  // stream-ordered: after the steps that read it
         b->d_tiles = nullptr;
         b->tiles_cap = 0;
-        CUDA_TRY(cudaMalloc(&b->d_tiles, sizeof(int2) * size_t(cap)));
+        // (of the contexts' pool: cudaMalloc took 0.7 ms of a new batch's first
+        // step for the 2.7 MB of 32 scenes)
+        CUDA_TRY(cudaMallocFromPoolAsync((void **)&b->d_tiles, sizeof(int2) * size_t(cap), pool, b->stream));
         b->tiles_cap = cap;
     }
     b->T.tile_list = b->d_tiles;
@@ -264,7 +267,7 @@ int mfree_batch_destroy(mfree_batch *b) {
             mfree_destroy(sl.c);
         }
     if (b->d_table) cudaFree(b->d_table);
-    if (b->d_tiles) cudaFree(b->d_tiles);
+    if (b->d_tiles) cudaFreeAsync(b->d_tiles, b->stream);
     for (auto e : b->timer)
         if (e) cudaEventDestroy(e);
     if (b->own_stream) cudaStreamDestroy(b->stream);

@@ -133,6 +133,8 @@ struct mfree_ctx {
 namespace mfree {
 namespace host {
 
+// the device's stream-ordered pool, which context memory comes from
+cudaMemPool_t context_pool(int dev);
 int default_tile_depth();
 int default_tile_cap(long long n, int num_sms);
 int hash_blocks(const mfree_ctx *c);
