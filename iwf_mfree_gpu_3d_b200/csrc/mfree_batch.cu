@@ -81,7 +81,8 @@ void drop_graph(mfree_batch *b) {
 bool live(const Slot &s) { return s.c != nullptr && s.status == 0; }
 
 // rebuild the device table for the running slots (stream-ordered upload;
-// the graph is dropped, it holds the old grid sizes)
+// the graph is dropped, it holds the old grid sizes).  The table stays dirty
+// when it fails: the old one may be gone, so the next step builds again.
 int build_table(mfree_batch *b, int record_every) {
     drop_graph(b);
     b->run.clear();
@@ -90,13 +91,14 @@ int build_table(mfree_batch *b, int record_every) {
     const int n = int(b->run.size());
     b->T.nscenes = n;
     b->table_record_every = record_every;
-    b->dirty = false;
+    b->dirty = n > 0;
     if (n == 0) return MFREE_OK;
     if (n > b->cap) {
         CUDA_TRY(cudaStreamSynchronize(b->stream));  // the old table may still be read
         if (b->d_table) cudaFree(b->d_table);
         b->d_table = nullptr;
         const int cap = std::max(n, 2 * b->cap);
+        b->cap = 0;
         CUDA_TRY(cudaMalloc(&b->d_table, table_bytes(cap)));
         b->cap = cap;
     }
@@ -120,8 +122,7 @@ int build_table(mfree_batch *b, int record_every) {
         mfree_ctx *c = sl.c;
         int st = ready(c);
         if (st) {
-            sl.status = st;
-            b->dirty = true;  // build again without it on the next call
+            sl.status = st;  // the next call builds without it
             return st;
         }
         sl.built = c->version;
@@ -165,6 +166,7 @@ int build_table(mfree_batch *b, int record_every) {
     CUDA_TRY(cudaMemcpyAsync(dint, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, b->stream));
     cudaError_t e = launch_interact_batch(b->T, b->cspm, b->cond, b->prec, 0, b->stream);
     if (e != cudaSuccess) return fail(MFREE_ERR_CUDA, std::string("batched pair kernel setup: ") + cudaGetErrorString(e));
+    b->dirty = false;
     return MFREE_OK;
 }
 
