@@ -36,10 +36,11 @@
 // read the last record of the current tile, so that the copies land while the
 // epilogue runs.
 //
-// What bounds it: instruction issue (half of the cycles) and shared-memory
-// wavefronts (55 %), with 16 warps an SM -- the registers and the staged halo
-// leave room for no more -- to hide latencies, and 29 % of warp time at the
-// tile's barriers; FP32 pipe 23 %, DRAM 3 % (ncu, 252,000 particles).  The split
+// What bounds it: instruction issue (52 % of the cycles) and shared-memory
+// wavefronts (57 %), with 16 warps an SM -- the registers and the staged halo
+// leave room for no more -- to hide latencies, and 25 % of warp time at the
+// tile's barriers; FP32 pipe 34 %, DRAM 5 % (profiles/kb_interact_1m.md, 1M
+// particles).  The split
 // follows from the instructions it saves: eight lanes a target throughout (an
 // earlier form) spent about 80 instruction slots a candidate on ballots and on
 // walking columns that are about as long as the group is wide.  Pair kernel,

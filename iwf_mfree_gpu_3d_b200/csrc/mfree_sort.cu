@@ -15,11 +15,13 @@
 // The sort is a stable counting sort: an atomic histogram of cell ids (and of
 // the scan's tiles), an exclusive scan (which is also the cell-range table the
 // pair loop reads), an atomic scatter, and a gather that takes each entry to
-// its rank by previous index within its cell.  Four kernels: for small scenes
-// the launches are what the sort costs (~3.5 us each; separate reduction, scan
-// of the tile sums and per-cell fix-up made it seven).  The result equals thrust's stable sort_by_key of
-// (cell id, 0..n-1): cells ascending, previous order inside a cell, blanked
-// particles (cell id INT_MAX in the reference) last in previous order.
+// its rank by previous index within its cell.  Four kernels (and a scan of the
+// tile sums on grids of many cells): for small scenes the launches are what the
+// sort costs (~3.5 us each; separate reduction, scan of the tile sums and
+// per-cell fix-up made it seven).  The result equals thrust's stable
+// sort_by_key of (cell id, 0..n-1): cells ascending, previous order inside a
+// cell, blanked particles (cell id INT_MAX in the reference) last in previous
+// order.
 // N stays on the device: no host round trip per step.
 #include "mfree_kernels.cuh"
 
