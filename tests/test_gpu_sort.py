@@ -105,17 +105,20 @@ def test_sparse_grid_in_a_batch():
 
 
 def test_scan_time_is_linear_in_the_cells():
-    # eight times the cells: 8 times the scan's work, or 64 times if each of its
-    # blocks added up all the tiles before it (at 640^3 cells 1.4 ms instead of 0.4)
+    # eight times the cells took 6.6 times as long, and 21 times while each of
+    # the scan's blocks added up all the tiles before it (0.43 and 1.43 ms)
     def ms(cells):
         sim = api.Simulation.from_scene(_sparse(cells))
         sim.step()
         sim.set_kernel_timing(True)
+        best = np.inf
         for _ in range(5):
+            sim.kernel_times()
             sim.step()
-        t = sim.kernel_times()
+            t = sim.kernel_times()
+            best = min(best, sum(t[k][0] for k in ("scan_reduce", "scan_top", "scan_down")))
         sim.close()
-        return sum(t[k][0] / max(t[k][1], 1) for k in ("scan_reduce", "scan_top", "scan_down"))
+        return best
 
     small, large = ms((320, 320, 320)), ms((640, 640, 640))
-    assert large < 20.0 * small, (small, large)
+    assert large < 12.0 * small, (small, large)
